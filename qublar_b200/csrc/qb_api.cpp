@@ -19,6 +19,7 @@
 #include "qb_internal.hpp"
 #include "qb_kernels.hpp"
 #include "qb_qubo.hpp"
+#include "qb_word.hpp"
 
 using namespace qb;
 
@@ -285,14 +286,21 @@ qb_status plan_ising(const qb_ising_desc* g, IsingPlan& P) {
     double sum_w2 = 0.0;
     P.w_min = 0;
     P.max_w = 0;
+    P.f0_sum = 0;
+    int64_t zeros = 0;
     for (int64_t e = 0; e < m; ++e) {
         const int64_t a = std::llabs(int64_t(g->ew[e]));
         sum_w2 += double(a) * double(a);
         P.max_w = std::max(P.max_w, a);
-        if (a != 0 && (P.w_min == 0 || a < P.w_min)) P.w_min = a;
+        P.f0_sum -= 2 * int64_t(g->ew[e]);
+        if (a == 0) ++zeros;
+        else if (P.w_min == 0 || a < P.w_min) P.w_min = a;
     }
+    P.one_size = zeros == 0 && P.w_min == P.max_w;
     P.B = 0;
+    P.max_deg = 0;
     for (int i = 0; i < n; ++i) {
+        P.max_deg = std::max(P.max_deg, int(row[size_t(i) + 1] - row[size_t(i)]));
         int64_t acc = 0;
         for (int64_t k = row[size_t(i)]; k < row[size_t(i) + 1]; ++k) acc += std::llabs(int64_t(w[size_t(k)]));
         P.B = std::max(P.B, acc);
@@ -330,7 +338,8 @@ qb_status plan_ising(const qb_ising_desc* g, IsingPlan& P) {
 // Device bytes upload_ising will take.
 int64_t ising_device_bytes(const IsingPlan& P) {
     return int64_t(P.row.size() + P.adj.size() + P.f0.size() + P.col.order.size() + P.col.class_ptr.size()) * 4 +
-           int64_t(P.wgt.size()) * P.weight_bytes + P.m * 12;
+           int64_t(P.wgt.size()) * P.weight_bytes + P.m * 12 +
+           (word_sweep(P) ? word_table_bytes(P) : 0);
 }
 
 qb_status upload_ising(IsingPlan& P, const qb_ising_desc* g, cudaStream_t st, int64_t* bytes) {
@@ -351,9 +360,10 @@ qb_status upload_ising(IsingPlan& P, const qb_ising_desc* g, cudaStream_t st, in
     if ((s = upload(P.d_eu, g->eu, size_t(P.m) * 4, st))) return s;
     if ((s = upload(P.d_ev, g->ev, size_t(P.m) * 4, st))) return s;
     if ((s = upload(P.d_ew, g->ew, size_t(P.m) * 4, st))) return s;
+    if (word_sweep(P) && (s = upload_words(P, st))) return s;
     QB_CUDA(cudaStreamSynchronize(st));
     *bytes = int64_t(P.d_row.bytes + P.d_adj.bytes + P.d_w.bytes + P.d_f0.bytes + P.d_order.bytes +
-                     P.d_class_ptr.bytes + P.d_eu.bytes + P.d_ev.bytes + P.d_ew.bytes);
+                     P.d_class_ptr.bytes + P.d_eu.bytes + P.d_ev.bytes + P.d_ew.bytes + P.d_wrec.bytes + P.d_wadj.bytes);
     return QB_OK;
 }
 
@@ -975,6 +985,7 @@ void qb::problem_release_device(qb_problem* p) {
     ResidualPlan& R = p->resid;
     QuboPlan& Q = p->qubo;
     DevBuf* all[] = {&I.d_row, &I.d_adj, &I.d_w, &I.d_f0, &I.d_order, &I.d_class_ptr, &I.d_eu, &I.d_ev, &I.d_ew,
+                     &I.d_wrec, &I.d_wadj,
                      &R.d_row, &R.d_ent, &R.d_lin, &R.d_q, &R.d_nbr_ptr, &R.d_nbr_home, &R.d_order, &R.d_class_ptr,
                      &R.d_chunks, &R.d_chunk_ptr, &R.d_d, &R.d_w64, &R.d_rrow, &R.d_rbit, &R.d_ra, &R.d_meta,
                      &R.d_nbr_new, &R.d_rbit_new, &R.d_o_row, &R.d_o_ray, &R.d_o_a, &R.d_o_nbr_ptr, &R.d_o_nbr,
@@ -1281,12 +1292,19 @@ extern "C" qb_status qb_solve(qb_problem* p, const qb_schedule* sch, uint32_t n_
             if ((s = alloc_async(r->d_f, size_t(R) * size_t(n) * 4, st))) return bail(s);
             if ((s = alloc_async(r->d_e_i64, size_t(R) * 8, st))) return bail(s);
             if ((s = alloc_async(r->d_e_scr, size_t(R) * 8, st))) return bail(s);
-            if (ising_smem_bytes(P) == 0 && (s = alloc_async(r->d_scratch, size_t(R) * size_t(n) * 5, st))) return bail(s);
+            if (ising_smem_bytes(P) == 0 && !(!b.trace && word_solve_fit(P, R)) &&
+                (s = alloc_async(r->d_scratch, size_t(R) * size_t(n) * 5, st))) return bail(s);
             b.f = r->d_f.as<int32_t>();
             b.e_i64 = r->d_e_i64.as<long long>();
             b.scratch = r->d_scratch.p;
             cudaEventRecord(r->ev0, st);
-            if ((s = launch_ising_anneal(P, b, R, r->sweeps, seed0, st))) return bail(s);
+            if (!b.trace && word_solve_fit(P, R)) {
+                AsyncAllocScope scope(st);
+                s = launch_word_solve(P, b.x, b.f, b.e_i64, b.temp, R, r->sweeps, seed0, r->d_tables, st);
+            } else {
+                s = launch_ising_anneal(P, b, R, r->sweeps, seed0, st);
+            }
+            if (s != QB_OK) return bail(s);
             cudaEventRecord(r->ev1, st);
             if ((s = launch_ising_energies(P, b.x, R, r->d_e_scr.as<long long>(), st))) return bail(s);
             if ((s = launch_i64_to_f64(r->d_e_scr.as<long long>(), R, b.e_f64, st))) return bail(s);
@@ -1486,7 +1504,7 @@ extern "C" void qb_result_destroy(qb_result* r) {
     cudaSetDevice(r->device);
     cudaStream_t st = r->stream;
     DevBuf* all[] = {&r->d_x, &r->d_f, &r->d_e_i64, &r->d_e_scr, &r->d_e_f64, &r->d_p, &r->d_temp, &r->d_drift,
-                     &r->d_accepts, &r->d_e_track, &r->d_scratch, &r->d_trace};
+                     &r->d_accepts, &r->d_e_track, &r->d_scratch, &r->d_tables, &r->d_trace};
     if (r->packed) qb_batch_destroy(r->packed);   // waits for the stream: its tables are in use until then
     for (DevBuf* b : all) free_async(*b, st);
     if (r->ev0) cudaEventDestroy(r->ev0);

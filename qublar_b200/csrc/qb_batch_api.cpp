@@ -12,6 +12,7 @@
 
 #include "qb_batch.hpp"
 #include "qb_internal.hpp"
+#include "qb_word.hpp"
 
 using namespace qb;
 
@@ -41,9 +42,9 @@ struct qb_batch {
     int64_t total_x = 0;
     int64_t total_r = 0;
     int64_t total_nnz = 0;
-    std::vector<IsingItem> h_items;
     std::vector<BatchInstDev> h_inst;
     DevBuf d_items, d_counter, d_x, d_f, d_e, d_p, d_temp, d_state, d_inst;
+    DevBuf d_witems, d_bundles;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
     bool synced = false;
 };
@@ -53,6 +54,14 @@ namespace {
 constexpr int kDefaultThreads = 512;
 constexpr int kDefaultSmem = 96 * 1024;
 constexpr int kDefaultGroup = 32;
+// Word units narrower than four replicas leave most of a pass's Philox lanes
+// to replicas that do not exist; the field-carrying kernel serves those.
+constexpr int kWordMinReplicas = 4;
+// The largest word unit, as a share of one SM's part of the whole batch: large
+// instances are split over their replicas until no unit outlasts the others
+// (128 mixed instances of 200 to 20,000 bits, 200 sweeps: 21.6 ms at 1.0, 25.7
+// at 0.6, 25.0 at 0.4: narrower units cost more instructions a proposal).
+constexpr double kWordUnitShare = 1.0;
 
 bool pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
 
@@ -159,7 +168,7 @@ qb_status prepare(const qb_batch_item* items, int32_t count, const qb_opts* opts
     if ((s = b->d_f.alloc(size_t(x_off) * 4))) return s;
     if ((s = b->d_e.alloc(size_t(e_off) * 8))) return s;
     if ((s = b->d_p.alloc(size_t(p_off) * 4))) return s;
-    if ((s = b->d_counter.alloc(sizeof(int)))) return s;
+    if ((s = b->d_counter.alloc(2 * sizeof(int)))) return s;
     if ((s = upload_vec(b->d_temp, temps, b->stream))) return s;
     b->h_inst.resize(b->inst.size());
     for (size_t k = 0; k < b->inst.size(); ++k)
@@ -178,17 +187,60 @@ struct Unit {
     double cost;
 };
 
+// A batch's launch tables: items of the field-carrying kernel, units of the
+// word kernel and their bundles.
+struct Work {
+    std::vector<IsingItem> items;
+    WordWork words;
+};
+
 // Splits every instance into replica groups for the shape `c`, sorts the
 // units largest first and writes their descriptors. sample > 0 replaces each
 // schedule by `sample` of its sweeps, evenly spaced (autotuning), read from
 // sample_temp (one table of `sample` entries per instance).
-qb_status build_items(qb_batch* b, const qb_batch_config& c, int sample, const double* sample_temp,
-                      std::vector<IsingItem>& out) {
+qb_status build_items(qb_batch* b, const qb_batch_config& c, bool smem_asked, int sample, const double* sample_temp,
+                      Work& work) {
+    std::vector<IsingItem>& out = work.items;
+    // instances of one coupling size run as words (qb_word.cu). A shared-memory
+    // bound that the caller gave is a bound on an instance's int32 state: one
+    // that exceeds it at a single replica runs on global state as asked.
+    const size_t word_cap = word_max_smem();
+    auto as_words = [&](const qb_batch::Inst& I) {
+        const IsingPlan& P = I.prob->ising;
+        return word_sweep(P) && I.R >= kWordMinReplicas && word_item_smem(P, 2) <= word_cap &&
+               !(smem_asked && batch_item_smem(I.n, 1) > size_t(c.smem_bytes));
+    };
+    double total = 0.0;
+    for (const qb_batch::Inst& I : b->inst)
+        if (as_words(I))
+            total += word_unit_cost(I.n, I.prob->ising.nnz, 16, sample > 0 ? sample : I.sweeps) * ((I.R + 31) / 32);
+    const double max_cost = kWordUnitShare * total / word_sms();
+    std::vector<WordUnit> wunits;
     std::vector<Unit> units;
     int64_t state_bytes = 0;
     for (size_t k = 0; k < b->inst.size(); ++k) {
         const qb_batch::Inst& I = b->inst[k];
         const IsingPlan& P = I.prob->ising;
+        if (as_words(I)) {
+            const int sweeps = sample > 0 ? sample : I.sweeps;
+            const int np = word_pairs(P, I.R, sweeps, max_cost);
+            for (int q0 = 0; q0 < I.R; q0 += 2 * np) {
+                WordUnit u;
+                word_fill(u.item, P, np, std::min(2 * np, I.R - q0), I.seed0 + uint64_t(q0));
+                u.item.temp = sample > 0 ? sample_temp + k * size_t(sample) : b->d_temp.as<double>() + I.temp_off;
+                u.item.sweep0 = 0;
+                u.item.sweep1 = sweeps;
+                u.item.flags = kItemInit | kItemFinal;
+                u.item.e_out = b->d_e.as<long long>() + I.e_off + q0;
+                u.item.x_out = b->d_x.as<uint8_t>() + I.x_off + int64_t(q0) * I.n;
+                u.item.f_out = b->d_f.as<int32_t>() + I.x_off + int64_t(q0) * I.n;
+                u.smem = word_item_smem(P, np);
+                u.cost = word_unit_cost(I.n, P.nnz, np, sweeps);
+                u.passes = word_class_passes(I.n, P.col.n_colours(), np);
+                wunits.push_back(u);
+            }
+            continue;
+        }
         int r0 = 0;
         while (r0 < I.R) {
             const int G0 = std::min(c.max_group, floor_pow2(I.R - r0));
@@ -248,21 +300,41 @@ qb_status build_items(qb_batch* b, const qb_batch_config& c, int sample, const d
         it.wbytes = P.weight_bytes;
     }
     b->global_items = n_global;
+    work.words = word_pack(wunits);
     return QB_OK;
 }
 
-qb_status run_items(qb_batch* b, const qb_batch_config& c, const std::vector<IsingItem>& items) {
+// The work tables to the device.
+qb_status upload_work(qb_batch* b, const Work& work) {
     qb_status s;
-    if ((s = b->d_items.alloc(items.size() * sizeof(IsingItem)))) return s;
-    QB_CUDA(cudaMemcpyAsync(b->d_items.p, items.data(), items.size() * sizeof(IsingItem), cudaMemcpyHostToDevice,
-                            b->stream));
-    BatchShape sh;
-    sh.threads = c.threads;
-    sh.smem_bytes = c.smem_bytes;
-    sh.ctas = c.ctas;
-    if (sh.ctas <= 0 && (s = batch_ctas(sh, &sh.ctas))) return s;
-    b->ctas = std::min<int>(sh.ctas, int(items.size()));
-    return launch_ising_batch(b->d_items.as<IsingItem>(), int(items.size()), b->d_counter.as<int>(), sh, b->stream);
+    if (!work.items.empty() && (s = upload_vec(b->d_items, work.items, b->stream))) return s;
+    if (!work.words.items.empty() && (s = upload_vec(b->d_witems, work.words.items, b->stream))) return s;
+    if (!work.words.items.empty() && (s = upload_vec(b->d_bundles, work.words.bundles, b->stream))) return s;
+    return QB_OK;
+}
+
+// One launch of each kind of item the batch has.
+qb_status launch_work(qb_batch* b, const qb_batch_config& c, const Work& work) {
+    qb_status s;
+    b->launches = 0;
+    b->ctas = 0;
+    if (!work.items.empty()) {
+        BatchShape sh{c.threads, c.smem_bytes, c.ctas};
+        if (sh.ctas <= 0 && (s = batch_ctas(sh, &sh.ctas))) return s;
+        b->ctas = std::min<int>(sh.ctas, int(work.items.size()));
+        if ((s = launch_ising_batch(b->d_items.as<IsingItem>(), int(work.items.size()), b->d_counter.as<int>(), sh,
+                                    b->stream)))
+            return s;
+        ++b->launches;
+    }
+    if (!work.words.items.empty()) {
+        b->ctas = std::max(b->ctas, std::min<int>(word_sms(), int(work.words.bundles.size())));
+        if ((s = launch_ising_words(work.words, b->d_witems.as<WordItem>(), b->d_bundles.as<WordBundle>(),
+                                    b->d_counter.as<int>(), b->stream)))
+            return s;
+        ++b->launches;
+    }
+    return QB_OK;
 }
 
 qb_status wait(qb_batch* b) {
@@ -297,6 +369,7 @@ extern "C" qb_status qb_batch_autotune(const qb_batch_item* items, int32_t count
         const int S = sample_sweeps ? sample_sweeps : 8;
         qb_batch* b = new (std::nothrow) qb_batch();
         if (!b) return fail(QB_ENOMEM, "qb_batch_autotune: out of host memory");
+        AsyncAllocScope scope(opts ? static_cast<cudaStream_t>(opts->stream) : nullptr, true);
         qb_status s = prepare(items, count, opts, b);
         if (s != QB_OK) {
             qb_batch_destroy(b);
@@ -331,14 +404,15 @@ extern "C" qb_status qb_batch_autotune(const qb_batch_item* items, int32_t count
         cudaEventCreate(&e0);
         cudaEventCreate(&e1);
         // time one shape on `its`; < 0 when it does not fit an SM
-        auto time_shape = [&](const qb_batch_config& c, const std::vector<IsingItem>& its, float* ms) -> qb_status {
+        auto time_shape = [&](const qb_batch_config& c, const Work& work, float* ms) -> qb_status {
             *ms = -1.0f;
             BatchShape sh{c.threads, c.smem_bytes, 0};
             int ctas = 0;
             if (batch_ctas(sh, &ctas) != QB_OK) return QB_OK;   // shape does not fit an SM
-            cudaEventRecord(e0, b->stream);
-            qb_status r = run_items(b, c, its);
+            qb_status r = upload_work(b, work);
             if (r != QB_OK) return r;
+            cudaEventRecord(e0, b->stream);
+            if ((r = launch_work(b, c, work)) != QB_OK) return r;
             cudaEventRecord(e1, b->stream);
             if (cudaEventSynchronize(e1) != cudaSuccess)
                 return cuda_fail(cudaGetLastError(), "cudaEventSynchronize", __FILE__, __LINE__);
@@ -352,8 +426,8 @@ extern "C" qb_status qb_batch_autotune(const qb_batch_item* items, int32_t count
             for (int sm : smem_c)
                 for (int g : group_c) {
                     qb_batch_config c{th, std::min(sm, cap), g, 0};
-                    std::vector<IsingItem> its;
-                    if ((s = build_items(b, c, S, d_st.as<double>(), its)) != QB_OK) break;
+                    Work its;
+                    if ((s = build_items(b, c, true, S, d_st.as<double>(), its)) != QB_OK) break;
                     float ms = 0.0f;
                     if ((s = time_shape(c, its, &ms)) != QB_OK) break;
                     if (ms >= 0.0f) timed.emplace_back(ms, c);
@@ -375,8 +449,8 @@ extern "C" qb_status qb_batch_autotune(const qb_batch_item* items, int32_t count
             DevBuf d_st4;
             s = upload_vec(d_st4, st4, b->stream);
             for (size_t q = 0; s == QB_OK && q < std::min<size_t>(3, timed.size()); ++q) {
-                std::vector<IsingItem> its;
-                if ((s = build_items(b, timed[q].second, S4, d_st4.as<double>(), its)) != QB_OK) break;
+                Work its;
+                if ((s = build_items(b, timed[q].second, true, S4, d_st4.as<double>(), its)) != QB_OK) break;
                 float ms = 0.0f;
                 if ((s = time_shape(timed[q].second, its, &ms)) != QB_OK) break;
                 if (ms >= 0.0f && (best < 0.0f || ms < best)) {
@@ -418,29 +492,26 @@ extern "C" qb_status qb_solve_batch(const qb_batch_item* items, int32_t count, c
             qb_batch_destroy(b);
             return e;
         };
+        // the batch's memory from the library's pool; qb_batch_destroy waits for the stream first
+        AsyncAllocScope scope(opts ? static_cast<cudaStream_t>(opts->stream) : nullptr, true);
         if ((s = prepare(items, count, opts, b)) != QB_OK) return bail(s);
         b->cfg = c;
-        if ((s = build_items(b, c, 0, nullptr, b->h_items)) != QB_OK) return bail(s);
-        b->work_items = int(b->h_items.size());
+        Work work;
+        if ((s = build_items(b, c, cfg && cfg->smem_bytes != 0, 0, nullptr, work)) != QB_OK) return bail(s);
+        b->work_items = int(work.items.size() + work.words.items.size());
         if (cudaEventCreate(&b->ev0) != cudaSuccess || cudaEventCreate(&b->ev1) != cudaSuccess ||
             cudaEventCreate(&b->ev2) != cudaSuccess)
             return bail(cuda_fail(cudaGetLastError(), "cudaEventCreate", __FILE__, __LINE__));
         // the descriptors go up before the timed region
-        if ((s = b->d_items.alloc(b->h_items.size() * sizeof(IsingItem)))) return bail(s);
-        QB_CUDA(cudaMemcpyAsync(b->d_items.p, b->h_items.data(), b->h_items.size() * sizeof(IsingItem),
-                                cudaMemcpyHostToDevice, b->stream));
-        BatchShape sh{c.threads, c.smem_bytes, c.ctas};
-        if (sh.ctas <= 0 && (s = batch_ctas(sh, &sh.ctas))) return bail(s);
-        b->ctas = std::min<int>(sh.ctas, b->work_items);
+        if ((s = upload_work(b, work)) != QB_OK) return bail(s);
         cudaEventRecord(b->ev0, b->stream);
-        if ((s = launch_ising_batch(b->d_items.as<IsingItem>(), b->work_items, b->d_counter.as<int>(), sh, b->stream)))
-            return bail(s);
+        if ((s = launch_work(b, c, work)) != QB_OK) return bail(s);
         cudaEventRecord(b->ev1, b->stream);
         if ((s = launch_batch_marginals(b->d_x.as<uint8_t>(), b->d_inst.as<BatchInstDev>(), int(b->inst.size()),
                                         b->total_bits, b->d_p.as<float>(), b->stream)))
             return bail(s);
         cudaEventRecord(b->ev2, b->stream);
-        b->launches = 2;
+        ++b->launches;
         *out = b;
         return QB_OK;
     });

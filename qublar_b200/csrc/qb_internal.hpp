@@ -195,6 +195,11 @@ struct IsingPlan {
     int64_t w_min = 0;
     double sigma = 0.0;
     int weight_bytes = 4;     // 1 (int8) or 4
+    int max_deg = 0;
+    bool one_size = false;    // every |w_ij| equals max_w (no zero weights)
+    int64_t f0_sum = 0;       // sum of the fields of x = 0: -2 sum_e w
+    // bytes per entry of d_wadj (indices of 2 n words)
+    int word_bytes() const { return n <= 32768 ? 2 : 4; }
     Colouring col;
     // host copies in sweep (new) order
     std::vector<int32_t> row;    // n + 1 (int32 offsets: nnz < 2^31 is required)
@@ -204,6 +209,7 @@ struct IsingPlan {
     // device
     DevBuf d_row, d_adj, d_w, d_f0, d_order, d_class_ptr;
     DevBuf d_eu, d_ev, d_ew;     // edge list as given (energy verifier)
+    DevBuf d_wrec, d_wadj;       // word sweep (word_sweep(p)): per-bit records, word indices of the neighbours
 };
 
 struct ResidualPlan {
@@ -324,6 +330,7 @@ struct qb_result {
     qb::DevBuf d_accepts;    // R accepted-flip counts (residual, qubo)
     qb::DevBuf d_e_track;    // R tracked energies minus offset (qubo)
     qb::DevBuf d_scratch;    // per-branch state that does not fit on chip
+    qb::DevBuf d_tables;     // word units and bundles of the launch (ising, many replicas)
     qb::DevBuf d_trace;      // R x sweeps: ising int64 tracked energies; residual, qubo fp64 per-sweep dE sums
     double trace_base = 0.0; // residual: energy of x = 0; qubo: the offset
     const int* d_err = nullptr;   // timeout flag of a cooperative sweep (inside d_scratch), or null

@@ -1,0 +1,101 @@
+"""The word sweep (graphs of one coupling size: replicas as the bits of a word)
+against the field-carrying sweeps and the oracle, bit for bit.
+
+Sizes sit where the kernel's index arithmetic can go wrong: degrees around the
+16 neighbours of a register, bits without neighbours, class tails, replica
+counts that do not fill a unit, couplings other than 1, and the two widths of
+the adjacency (32,768 bits).
+"""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from qublar_b200 import Budget, IsingProblem, solve_batch, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _star_graph(n, degrees, w, seed):
+    """Bit k of the first len(degrees) has degrees[k] neighbours of its own
+    among the rest; the remaining bits have at most one."""
+    rng = np.random.default_rng(seed)
+    eu, ev, at = [], [], len(degrees)
+    for k, d in enumerate(degrees):
+        eu += [k] * d
+        ev += list(range(at, at + d))
+        at += d
+    assert at <= n
+    return n, np.array(eu, np.int32), np.array(ev, np.int32), (w * rng.choice([-1, 1], len(eu))).astype(np.int32)
+
+
+GRAPHS = {
+    "degrees": lambda: _star_graph(400, [0, 1, 15, 16, 17, 31, 32, 33, 47, 48, 49, 64], 1, 3),
+    "w7": lambda: (lambda g: (g[0], g[1], g[2], 7 * g[3]))(synth.random_regular(203, 9, 5)),
+    "torus": lambda: synth.torus_pm1(19, 8),
+    "dense": lambda: synth.erdos_renyi(90, 0.6, 4),
+    "two": lambda: (2, np.array([0], np.int32), np.array([1], np.int32), np.array([-3], np.int32)),
+}
+
+
+@pytest.mark.parametrize("R", [4, 7, 16, 33, 70])
+@pytest.mark.parametrize("name", list(GRAPHS))
+def test_words_equal_the_oracle(name, R):
+    g = GRAPHS[name]()
+    P = IsingProblem(*g)
+    s = P.scaled_schedule(30, 4)
+    B = solve_batch([(P, s, R, 6)])
+    X, E, F = B.branches(0), B.energies_tracked(0), B.fields(0)
+    G = O.Graph(*g)
+    order, _ = P.colouring()
+    temps = O.temperatures(s.t_hot, s.t_cold, s.anneal_sweeps, s.hold_sweeps)
+    for r in sorted({0, 1, R // 2, R - 1}):
+        key, half = O.ising_key_half(r, 6)
+        x, f, e = G.anneal_coloured(order, temps, key, half=half)
+        assert (X[r] == x).all() and E[r] == e, r
+    for r in range(R):
+        assert E[r] == -G.cut(X[r]) and (F[r] == G.fields(X[r])).all()
+    B.close()
+
+
+@pytest.mark.parametrize("R", [32, 29, 16, 8, 4])
+@pytest.mark.parametrize("name", ["degrees", "w7", "torus"])
+def test_every_unit_width_equals_the_oracle(name, R):
+    """Enough instances that none is split: units of 32, 16, 8 and 4 replicas."""
+    g = GRAPHS[name]()
+    P = IsingProblem(*g)
+    s = P.scaled_schedule(12, 2)
+    B = solve_batch([(P, s, R, 64 * k) for k in range(700)])
+    assert B.info().work_items == 700
+    G = O.Graph(*g)
+    order, _ = P.colouring()
+    temps = O.temperatures(s.t_hot, s.t_cold, s.anneal_sweeps, s.hold_sweeps)
+    for k in (0, 311, 699):
+        X, E, F = B.branches(k), B.energies_tracked(k), B.fields(k)
+        for r in range(R):
+            key, half = O.ising_key_half(r, 64 * k)
+            x, f, e = G.anneal_coloured(order, temps, key, half=half)
+            assert (X[r] == x).all() and E[r] == e and (F[r] == f).all(), (k, r)
+    B.close()
+
+
+@pytest.mark.parametrize("n", [32767, 32769])
+def test_both_adjacency_widths_equal_the_field_sweep(n):
+    g = synth.random_regular(n, 5, 11)
+    P = IsingProblem(*g)
+    s = P.scaled_schedule(8, 1)
+    B = solve_batch([(P, s, 10, 0)])
+    r = P.solve(s, 10)
+    assert (B.branches(0) == r.branches()).all()
+    assert (B.energies_tracked(0) == r.energies_tracked()).all() and (B.fields(0) == r.fields()).all()
+
+
+@pytest.mark.parametrize("R", [149, 301, 1200])
+def test_many_replicas_equal_the_cta_per_replica_sweep(R, monkeypatch):
+    g = synth.random_regular(331, 21, 2)
+    P = IsingProblem(*g)
+    b = Budget(6.0, 0.2, 40, 3)
+    r = P.solve(b, R, 4)
+    monkeypatch.setenv("QB_ISING_THREADS", "128")
+    o = P.solve(b, R, 4)
+    assert (r.branches() == o.branches()).all() and (r.fields() == o.fields()).all()
+    assert (r.energies_tracked() == o.energies_tracked()).all() and (r.energies() == o.energies()).all()
