@@ -1215,6 +1215,11 @@ extern "C" qb_status qb_schedule_scaled(const qb_problem* p, int32_t anneal_swee
 
 // ---- solve ---------------------------------------------------------------------------------------
 
+// The sweep an ising solve takes (all give the same branches): few replicas
+// and dense graphs (qb_replica.cu), many replicas of one coupling size
+// (qb_word.cu), otherwise a CTA per replica with its fields (qb_kernels.cu).
+enum class IsingRoute { kReplicas, kWords, kFields };
+
 extern "C" qb_status qb_solve(qb_problem* p, const qb_schedule* sch, uint32_t n_branches, uint64_t seed_offset,
                               const qb_opts* opts, qb_result** out) {
     return qb::guarded("qb_solve", [&]() -> qb_status {
@@ -1292,13 +1297,18 @@ extern "C" qb_status qb_solve(qb_problem* p, const qb_schedule* sch, uint32_t n_
             if ((s = alloc_async(r->d_f, size_t(R) * size_t(n) * 4, st))) return bail(s);
             if ((s = alloc_async(r->d_e_i64, size_t(R) * 8, st))) return bail(s);
             if ((s = alloc_async(r->d_e_scr, size_t(R) * 8, st))) return bail(s);
-            if (ising_smem_bytes(P) == 0 && !(!b.trace && word_solve_fit(P, R)) &&
+            const IsingRoute route = replica_solve_fit(P, R, std::max(sch->t_hot, sch->t_cold)) ? IsingRoute::kReplicas
+                                     : !b.trace && word_solve_fit(P, R)                        ? IsingRoute::kWords
+                                                                                               : IsingRoute::kFields;
+            if (route == IsingRoute::kFields && ising_smem_bytes(P) == 0 &&
                 (s = alloc_async(r->d_scratch, size_t(R) * size_t(n) * 5, st))) return bail(s);
             b.f = r->d_f.as<int32_t>();
             b.e_i64 = r->d_e_i64.as<long long>();
             b.scratch = r->d_scratch.p;
             cudaEventRecord(r->ev0, st);
-            if (!b.trace && word_solve_fit(P, R)) {
+            if (route == IsingRoute::kReplicas) {
+                s = launch_ising_replicas(P, b, R, r->sweeps, seed0, st);
+            } else if (route == IsingRoute::kWords) {
                 AsyncAllocScope scope(st);
                 s = launch_word_solve(P, b.x, b.f, b.e_i64, b.temp, R, r->sweeps, seed0, r->d_tables, st);
             } else {

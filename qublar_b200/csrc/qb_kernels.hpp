@@ -31,6 +31,11 @@ struct SolveBuffers {
 size_t ising_smem_bytes(const IsingPlan& p);
 qb_status launch_ising_anneal(const IsingPlan& p, const SolveBuffers& b, int R, int sweeps, uint64_t seed0,
                               cudaStream_t st);
+// At most one replica per SM: the sweep with the draws off its chain
+// (qb_replica.cu); t_max: the schedule's largest temperature.
+bool replica_solve_fit(const IsingPlan& p, int R, double t_max);
+qb_status launch_ising_replicas(const IsingPlan& p, const SolveBuffers& b, int R, int sweeps, uint64_t seed0,
+                                cudaStream_t st);
 qb_status launch_ising_energies(const IsingPlan& p, const uint8_t* x, int K, long long* e, cudaStream_t st);
 
 size_t resid_smem_bytes(const ResidualPlan& p);

@@ -1,0 +1,73 @@
+"""The few-replica integer sweep (draws reduced to the largest accepted dE,
+off the sweep's chain) against the CTA-per-replica sweep and the oracle, bit
+for bit: tiny and wide classes, a warp per flip and a lane per flip, helper
+CTAs, an adjacency too large for shared memory, couplings from 1 to 10^6 (both
+precisions of the limit's logarithm), and the per-sweep trace."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from qublar_b200 import IsingProblem, Schedule, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _sparse(n, m, wmax, seed):
+    rng = np.random.default_rng(seed)
+    keys = np.unique(rng.integers(0, n, 2 * m) * n + rng.integers(0, n, 2 * m))
+    u, v = keys // n, keys % n
+    keep = u < v
+    u, v = u[keep][:m], v[keep][:m]
+    w = rng.integers(1, wmax + 1, u.size) * rng.choice([-1, 1], u.size)
+    return n, u.astype(np.int32), v.astype(np.int32), w.astype(np.int32)
+
+
+CASES = {
+    "k16": (lambda: synth.random_complete(16, 15, 3), 32, 60),
+    "two": (lambda: (2, np.array([0], np.int32), np.array([1], np.int32), np.array([5], np.int32)), 3, 20),
+    "er": (lambda: synth.erdos_renyi(300, 0.16, 2), 5, 80),
+    "dense_1000": (lambda: synth.random_complete(121, 1000, 7), 4, 60),
+    "dense_1e6": (lambda: synth.random_complete(65, 1000000, 7), 4, 60),
+    "dense_33": (lambda: synth.random_complete(33, 7, 1), 200, 30),
+    "dense_128": (lambda: synth.random_complete(128, 1, 2), 3, 30),
+    "dense_224": (lambda: synth.random_complete(224, 500, 2), 3, 17),
+    "dense_225": (lambda: synth.random_complete(225, 500, 2), 3, 9),
+    "torus": (lambda: synth.torus_pm1(30, 3), 7, 50),
+    "dense_many": (lambda: synth.random_complete(50, 1, 3), 700, 20),
+    "sparse_helpers": (lambda: _sparse(3001, 12000, 900, 5), 3, 40),
+    "sparse_many": (lambda: _sparse(2001, 9000, 100, 6), 100, 20),
+    "long_rows": (lambda: _sparse(9001, 180000, 3, 8), 2, 8),
+}
+
+
+@pytest.mark.parametrize("name", list(CASES))
+def test_equals_the_cta_per_replica_sweep_and_the_oracle(name, monkeypatch):
+    make, R, sweeps = CASES[name]
+    g = make()
+    P = IsingProblem(*g)
+    s = P.scaled_schedule(sweeps, 3)
+    r = P.solve(s, R, 9, trace=True)
+    monkeypatch.setenv("QB_ISING_THREADS", "512")
+    o = P.solve(s, R, 9, trace=True)
+    monkeypatch.delenv("QB_ISING_THREADS")
+    assert (r.branches() == o.branches()).all() and (r.fields() == o.fields()).all()
+    assert (r.energies_tracked() == o.energies_tracked()).all() and (r.energies() == o.energies()).all()
+    assert (r.energy_trace() == o.energy_trace()).all()
+    G = O.Graph(*g)
+    order, _ = P.colouring()
+    temps = O.temperatures(s.t_hot, s.t_cold, s.anneal_sweeps, s.hold_sweeps)
+    for k in (0, R - 1):
+        key, half = O.ising_key_half(k, 9)
+        x, f, e = G.anneal_coloured(order, temps, key, half=half)
+        assert (r.branches()[k] == x).all() and r.energies_tracked()[k] == e
+
+
+@pytest.mark.parametrize("t", [1e-3, 0.7, 4095.0, 4097.0, 3e7, 1e13, 1e16])
+def test_temperatures_of_every_size(t, monkeypatch):
+    g = synth.random_complete(40, 20000, 1)
+    P = IsingProblem(*g)
+    s = Schedule(t, t / 3, 25, 2, 0)
+    r = P.solve(s, 6)
+    monkeypatch.setenv("QB_ISING_THREADS", "64")
+    o = P.solve(s, 6)
+    assert (r.branches() == o.branches()).all() and (r.energies_tracked() == o.energies_tracked()).all()
