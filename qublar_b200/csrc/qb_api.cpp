@@ -18,6 +18,7 @@
 #include "qb_batch.hpp"
 #include "qb_internal.hpp"
 #include "qb_kernels.hpp"
+#include "qb_local.hpp"
 #include "qb_qubo.hpp"
 #include "qb_word.hpp"
 
@@ -717,6 +718,11 @@ qb_status plan_residual(const qb_residual_desc* d, ResidualPlan& P, int lock_sli
         P.chunk_ptr[size_t(t) + 1] = int32_t(P.chunks.size() / 8);
     }
     mark("chunks");
+    P.local = lock && resid_local_fit(n, nr, nc);
+    if (P.local) {
+        resid_local_plan(P);
+        mark("local items");
+    }
     mark.print();
     return QB_OK;
 }
@@ -732,6 +738,7 @@ int64_t residual_device_bytes(const ResidualPlan& P) {
                         P.h_nbr_home.size() + P.col.order.size() + P.col.class_ptr.size() + P.chunks.size() +
                         P.chunk_ptr.size()) * 4;
     b += (nr + 1) * 4 + nnz * 12 + n * 8 + nr * 16 + (n + 1) * 4 + P.n_nbr * 4;   // ray-major CSR (two bit orders)
+    if (P.local) b += int64_t(P.l_rec.size() + P.l_ptr.size()) * 4;
     if (P.variant == QB_RESID_LOCKSTEP) b += int64_t(P.h_meta.size() + P.h_nbr_new.size()) * 4 + nnz * 4;
     return b;
 }
@@ -882,6 +889,9 @@ qb_status upload_residual(ResidualPlan& P, const qb_residual_desc* d, cudaStream
     if (lock) {
         QB_UP(d_meta, P.h_meta); QB_UP(d_nbr_new, P.h_nbr_new);
     }
+    if (P.local) {
+        QB_UP(d_lrec, P.l_rec); QB_UP(d_lptr, P.l_ptr);
+    }
 #undef QB_UP
     if ((s = upload(P.d_d, d->d, size_t(nr) * 8, st))) return s;
     if ((s = upload(P.d_o_nbr_ptr, d->nbr_ptr, (size_t(n) + 1) * 4, st))) return s;
@@ -890,7 +900,7 @@ qb_status upload_residual(ResidualPlan& P, const qb_residual_desc* d, cudaStream
     const DevBuf* all[] = {&P.d_row, &P.d_ent, &P.d_lin, &P.d_q, &P.d_nbr_ptr, &P.d_nbr_home, &P.d_order,
                            &P.d_class_ptr, &P.d_chunks, &P.d_chunk_ptr, &P.d_d, &P.d_w64, &P.d_rrow, &P.d_rbit,
                            &P.d_ra, &P.d_o_rbit, &P.d_o_nbr_ptr, &P.d_o_nbr, &P.d_o_lin,
-                           &P.d_meta, &P.d_nbr_new, &P.d_rbit_new};
+                           &P.d_meta, &P.d_nbr_new, &P.d_rbit_new, &P.d_lrec, &P.d_lptr};
     int64_t tot = 0;
     for (const DevBuf* b : all) tot += int64_t(b->bytes);
     *bytes = tot;
@@ -989,7 +999,7 @@ void qb::problem_release_device(qb_problem* p) {
                      &R.d_row, &R.d_ent, &R.d_lin, &R.d_q, &R.d_nbr_ptr, &R.d_nbr_home, &R.d_order, &R.d_class_ptr,
                      &R.d_chunks, &R.d_chunk_ptr, &R.d_d, &R.d_w64, &R.d_rrow, &R.d_rbit, &R.d_ra, &R.d_meta,
                      &R.d_nbr_new, &R.d_rbit_new, &R.d_o_row, &R.d_o_ray, &R.d_o_a, &R.d_o_nbr_ptr, &R.d_o_nbr,
-                     &R.d_o_lin, &R.d_o_rbit,
+                     &R.d_o_lin, &R.d_o_rbit, &R.d_lrec, &R.d_lptr,
                      &Q.d_row, &Q.d_adj, &Q.d_J, &Q.d_h, &Q.d_order, &Q.d_class_ptr, &Q.d_eu, &Q.d_ev, &Q.d_ew, &Q.d_ho,
                      &p->d_temp};
     // buffers of the plain create path go back to the pool on the legacy
@@ -1360,7 +1370,8 @@ extern "C" qb_status qb_solve(qb_problem* p, const qb_schedule* sch, uint32_t n_
             b.drift = r->d_drift.as<float>();
             b.accepts = r->d_accepts.as<unsigned long long>();
             const int RB = std::min(R, resid_lockstep_max_branches());   // branches per lockstep launch
-            if (P.variant == QB_RESID_LOCKSTEP) {
+            const bool local = resid_local_route(P);
+            if (P.variant == QB_RESID_LOCKSTEP && !local) {
                 if ((s = alloc_async(r->d_scratch, resid_lockstep_scratch(P, RB), st))) return bail(s);
                 b.scratch = r->d_scratch.p;
                 QB_CUDA(cudaMemsetAsync(r->d_scratch.p, 0, 64, st));   // control block, timeout flag included
@@ -1368,7 +1379,10 @@ extern "C" qb_status qb_solve(qb_problem* p, const qb_schedule* sch, uint32_t n_
             }
             cudaEventRecord(r->ev0, st);
             int anneal_launches = 0;
-            if (P.variant == QB_RESID_LOCKSTEP) {
+            if (local) {
+                s = launch_resid_local(P, b, R, r->sweeps, sch->refresh_sweeps, seed0, st);
+                anneal_launches = 1;
+            } else if (P.variant == QB_RESID_LOCKSTEP) {
                 // blocks of at most RB branches, one cooperative launch each
                 for (int b0 = 0; b0 < R && s == QB_OK; b0 += RB, ++anneal_launches) {
                     SolveBuffers bb = b;

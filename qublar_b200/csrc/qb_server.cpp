@@ -26,6 +26,7 @@
 #include "qb_batch.hpp"
 #include "qb_internal.hpp"
 #include "qb_kernels.hpp"
+#include "qb_local.hpp"
 #include "qb_qubo.hpp"
 
 using namespace qb;
@@ -349,7 +350,8 @@ qb_status launch_coop(qb_server* S, Request* r, cudaStream_t st, int qubo_ctas) 
         if ((s = launch_qubo_energies(r->prob->qubo, x, r->R, r->d_ef64.as<double>(), st))) return s;
     } else {
         const ResidualPlan& P = r->prob->resid;
-        const int RB = resid_lockstep_max_branches();
+        const bool local = resid_local_route(P);
+        const int RB = local ? r->R : resid_lockstep_max_branches();
         for (int b0 = 0; b0 < r->R; b0 += RB) {
             SolveBuffers b;
             b.x = x + size_t(b0) * size_t(r->n);
@@ -357,9 +359,10 @@ qb_status launch_coop(qb_server* S, Request* r, cudaStream_t st, int qubo_ctas) 
             b.drift = r->d_drift.as<float>() + b0;
             b.accepts = r->d_accepts.as<unsigned long long>() + b0;
             b.scratch = r->d_state.p;
-            if ((s = launch_resid_lockstep(P, b, std::min(RB, r->R - b0), r->sweeps, r->sched.refresh_sweeps,
-                                           r->seed0 + uint64_t(b0), st)))
-                return s;
+            if (local) s = launch_resid_local(P, b, r->R, r->sweeps, r->sched.refresh_sweeps, r->seed0, st);
+            else s = launch_resid_lockstep(P, b, std::min(RB, r->R - b0), r->sweeps, r->sched.refresh_sweeps,
+                                           r->seed0 + uint64_t(b0), st);
+            if (s != QB_OK) return s;
         }
         if ((s = launch_resid_energies(P, x, r->R, r->d_ef64.as<double>(), st))) return s;
     }

@@ -1,0 +1,68 @@
+"""The residual sweep with a CTA per branch against the lockstep sweep and the
+oracle, bit for bit: empty and single rays, bits without rays, bits of one to
+more than sixteen segments, more branches than SMs, negative weights, long
+neighbour lists, the refresh, traces."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from qublar_b200 import ResidualProblem, Schedule, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _random(n, rays, degrees, seed, nbrs=3):
+    """Bits with the given numbers of rays (cycled), a ring of neighbours, some negative weights."""
+    rng = np.random.default_rng(seed)
+    row, ray, a = [0], [], []
+    for i in range(n):
+        k = min(rays, degrees[i % len(degrees)])
+        ray += list(rng.choice(rays, k, replace=False))
+        a += list(rng.uniform(0.05, 0.4, k))
+        row.append(len(ray))
+    nb = [[] for _ in range(n)]
+    for i in range(n):
+        for s in range(1, nbrs + 1):
+            j = (i + s) % n
+            if j != i and j not in nb[i]:
+                nb[i].append(j)
+                nb[j].append(i)
+    ptr = np.cumsum([0] + [len(v) for v in nb])
+    w = rng.uniform(0.5, 3.0, rays) * rng.choice([1.0, 1.0, 1.0, -1.0], rays)
+    return {"d": rng.uniform(0.0, 1.0, rays), "w": w, "row_ptr": np.array(row, np.int32),
+            "ray": np.array(ray, np.int32), "a": np.array(a, np.float32), "nbr_ptr": ptr.astype(np.int32),
+            "nbr": np.array([j for v in nb for j in v], np.int32), "lambda": 0.3, "kappa": 0.4, "field": None}
+
+
+CASES = {
+    "exhaustive16": (synth.exhaustive16, 20, 60),
+    "pyramid": (lambda: synth.tomography(synth.small_tomo_params(0.16, 16)), 9, 70),
+    "edges": (lambda: _random(230, 600, [0, 1, 2, 15, 16, 17, 31, 32, 33, 48, 200, 255, 256, 257, 300, 530], 4), 5, 25),
+    "one_ray": (lambda: _random(12, 1, [1, 0], 2, 1), 3, 30),
+    "long_neighbours": (lambda: _random(90, 40, [3, 20], 6, 14), 4, 40),
+    "many_branches": (lambda: _random(60, 30, [4, 9], 7), 331, 30),
+}
+
+
+@pytest.mark.parametrize("name", list(CASES))
+def test_equals_the_lockstep_sweep_and_the_oracle(name, monkeypatch):
+    make, R, sweeps = CASES[name]
+    arr = make()
+    P = ResidualProblem.from_arrays(arr)
+    s = Schedule(20.0, 0.6, sweeps, 6, 11)
+    r = P.solve(s, R, 3, trace=True)
+    monkeypatch.setenv("QB_RESID_KERNEL", "lockstep")
+    o = P.solve(s, R, 3, trace=True)
+    monkeypatch.delenv("QB_RESID_KERNEL")
+    X = r.branches()
+    assert (X == o.branches()).all() and (r.marginals() == o.marginals()).all()
+    assert np.array_equal(r.energies(), o.energies())
+    a, b = r.info(), o.info()
+    assert a.accepted == b.accepted and a.max_drift == b.max_drift
+    scale = np.maximum(1.0, np.abs(o.energy_trace()).max())
+    assert np.abs(r.energy_trace() - o.energy_trace()).max() <= 1e-12 * sweeps * scale   # fp64 sums in another order
+    order, _ = P.colouring()
+    temps = O.temperatures(s.t_hot, s.t_cold, s.anneal_sweeps, s.hold_sweeps)
+    for k in (0, R - 1):
+        x, _ = O.resid_anneal_coloured(arr, order, temps, s.refresh_sweeps, k + 4, mode=1)
+        assert (X[k] == x).all(), k
