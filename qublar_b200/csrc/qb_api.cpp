@@ -1370,7 +1370,7 @@ extern "C" qb_status qb_solve(qb_problem* p, const qb_schedule* sch, uint32_t n_
             b.drift = r->d_drift.as<float>();
             b.accepts = r->d_accepts.as<unsigned long long>();
             const int RB = std::min(R, resid_lockstep_max_branches());   // branches per lockstep launch
-            const bool local = resid_local_route(P);
+            const bool local = resid_local_route(P, R);
             if (P.variant == QB_RESID_LOCKSTEP && !local) {
                 if ((s = alloc_async(r->d_scratch, resid_lockstep_scratch(P, RB), st))) return bail(s);
                 b.scratch = r->d_scratch.p;

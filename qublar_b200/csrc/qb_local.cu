@@ -4,21 +4,26 @@
 // The lockstep sweep (qb_kernels.cu) keeps all branches in global memory and
 // closes every colour class with a grid barrier: about 4 us a class step
 // whatever the class holds. Branches do not interact, so a branch that fits one
-// SM needs no grid at all: a class step is gathers from shared memory and one
-// CTA barrier.
+// SM needs no grid at all: a class step is gathers from shared memory and a
+// barrier of the warps that take part.
 //
 // A warp item is 16 lane pairs, a pair per 16-entry segment of a bit (the even
 // and the odd entries' fmaf chains, as in the lockstep sweep), a bit's pairs
 // side by side: its segment sums are added in order through shuffles, every
 // lane of the bit takes the decision, and each lane updates the residuals it
 // holds -- no block barrier inside a class. A bit of more than 16 segments
-// takes a warp to itself and goes over its segments in rounds. A warp's next
-// item (record, entries, neighbour list, draw) is loaded while the current one
-// runs; none of it depends on the state.
+// takes a warp to itself and goes over its segments in rounds. What does not
+// depend on the state (record, entries, neighbour list, draw) is loaded and
+// computed for a warp's next item as soon as it has finished one; items are
+// dealt to the warps in a row over all classes, so that is a class or more
+// ahead of its use.
 //
-// Bound: the class step's chain (about 0.4 us) on small problems, the random
-// 8-byte gathers from shared memory (about 5 lanes a cycle and SM, measured) on
-// large ones.
+// Bound: the dependent instructions of an item in its warp (about 1 us a class
+// step; loads and draws are off it), on larger problems the items per SM.
+// Measured on a B200, 100 sweeps: 5,020 bits, 24 branches 34.9 ms lockstep,
+// 10.2 here (12.9 with the next item's loads ahead of a CTA-wide barrier, 11.6
+// with items dealt in turn, 10.2 with barriers of the two classes' warps only);
+// 20,000 bits, 16 branches 52 and 31; 40,000 bits, 64 branches 83 and 54.
 //
 // The arithmetic, the draws and hence the branches are the lockstep sweep's.
 #include <cuda_runtime.h>
@@ -38,7 +43,7 @@ namespace qb {
 namespace {
 
 constexpr unsigned kAllLanes = 0xffffffffu;
-constexpr int kLocalThreads = 512;
+constexpr int kLocalThreads = 480;   // 15 warps: see the class barriers
 constexpr int kLocalWarps = kLocalThreads / 32;
 constexpr int kPairs = 16;          // segments per warp item
 constexpr int kSegE = 16;           // entries per segment
@@ -76,9 +81,6 @@ struct ResidLocalArgs {
 // of its bit << 5 | length of the bit's last segment << 10 | the bit's segments
 // << 16 (0: empty pair); the bit's sweep position; its input index; lin, q,
 // first neighbour, neighbours.
-struct Rec {
-    uint4 a, b;
-};
 __host__ __device__ inline uint32_t rec_tag(int len, int pair, int last, int segs) {
     return uint32_t(len) | uint32_t(pair) << 5 | uint32_t(last) << 10 | uint32_t(segs) << 16;
 }
@@ -89,7 +91,7 @@ __global__ void __launch_bounds__(kLocalThreads, 1) resid_local_kernel(ResidLoca
     __shared__ unsigned long long s_accepts;
     const int nr = A.n_rays, n = A.n, nc = A.n_colours, words = (n + 31) / 32;
     float2* rho = reinterpret_cast<float2*>(smem);
-    uint32_t* xs = reinterpret_cast<uint32_t*>(rho + nr);
+    uint32_t* xs = reinterpret_cast<uint32_t*>(rho + nr + 1);
     int32_t* ip = reinterpret_cast<int32_t*>(xs + words);
     const int tid = int(threadIdx.x), lane = tid & 31;
     const int warp = __shfl_sync(kAllLanes, tid >> 5, 0);
@@ -98,6 +100,7 @@ __global__ void __launch_bounds__(kLocalThreads, 1) resid_local_kernel(ResidLoca
     const uint64_t seed = A.seed0 + uint64_t(branch);
     for (int b = tid; b < nr; b += kLocalThreads) rho[b] = split_pair(-__dmul_rn(sqrt(fabs(A.w64[b])), A.d[b]));
     for (int k = tid; k < words; k += kLocalThreads) xs[k] = 0u;
+    if (tid == 0) rho[nr] = make_float2(0.0f, 0.0f);
     for (int c = tid; c <= nc; c += kLocalThreads) ip[c] = __ldg(A.item_ptr + c);
     if (tid == 0) {
         s_trace = 0.0;
@@ -106,113 +109,148 @@ __global__ void __launch_bounds__(kLocalThreads, 1) resid_local_kernel(ResidLoca
     __syncthreads();
 
     auto bit_of = [&](int i) { return (xs[i >> 5] >> (i & 31)) & 1u; };
-    auto rec_of = [&](int it) {
-        const uint4* r = A.rec + (size_t(it) * kPairs + size_t(pair)) * 2;
-        return Rec{__ldg(r), __ldg(r + 1)};
-    };
-    // the warp's items in visiting order: the next one of this class, else the
-    // first of the next class that has one for it
-    auto advance = [&](int& c, int& it, int& sweep) {
-        it += kLocalWarps;
-        if (it < ip[c + 1]) return;
-        for (int k = 0; k < nc; ++k) {
-            if (++c == nc) {
-                c = 0;
-                ++sweep;
-            }
-            it = ip[c] + warp;
-            if (it < ip[c + 1]) return;
+    // The items of all classes in a row are dealt to the warps in turn, so a
+    // warp's next item lies a class or more ahead and its loads and draw run
+    // while other warps have the current class.
+    const int total = ip[nc];
+    int c0 = 0, it0 = warp, s0 = 0;
+    auto settle = [&]() {   // the class of item it0 (of a later sweep past the end)
+        while (it0 >= total) {
+            it0 -= total;
+            ++s0;
+            c0 = 0;
         }
-        sweep = A.sweeps;   // no item at all
+        while (it0 >= ip[c0 + 1]) ++c0;
     };
-    // what an item loads ahead besides its record
-    uint2 ent[kHold];
-    int nb[kNbrLane];
+    auto rec_of = [&](int it) { return A.rec + (size_t(it) * kPairs + size_t(pair)) * 2; };
+    // The item in hand: its record, and per entry of the lane its residual and
+    // coefficient; entries past the segment are the zero pair rho[nr] with a
+    // zero coefficient, which change nothing. na, nb: the next item's record.
+    // issue() starts the loads and makes the draw, nothing in it waits for
+    // them: it runs ahead of the barrier, whose wait hides them.
+    uint4 ra{}, rb{}, na{}, nb{};
+    uint2 en[kHold];
+    int nbr[kNbrLane];
     uint64_t u53 = 0;
-    auto fetch = [&](const Rec& r, int sweep) {
-        const int len = int(r.a.y & 31u);
+    auto issue = [&]() {
+        ra = na;
+        rb = nb;
+        int ni = it0 + kLocalWarps;
+        while (ni >= total) ni -= total;
+        const uint4* next = rec_of(ni);
+        na = __ldg(next);
+        nb = __ldg(next + 1);
+        const int len = int(ra.y & 31u);
 #pragma unroll
         for (int u = 0; u < kHold; ++u) {
-            ent[u] = make_uint2(0u, 0u);
-            if (half + 2 * u < len) ent[u] = __ldg(A.ent + r.a.x + half + 2 * u);
+            en[u] = make_uint2(uint32_t(nr), 0u);
+            if (half + 2 * u < len) en[u] = __ldg(A.ent + ra.x + half + 2 * u);
         }
         // lanes 0 and 1 of the bit share its neighbours
-        const int gl = lane - 2 * int((r.a.y >> 5) & 31u);
+        const int gl = lane - 2 * int((ra.y >> 5) & 31u);
 #pragma unroll
         for (int t = 0; t < kNbrLane; ++t)
-            nb[t] = (r.a.y >> 16) && gl < 2 && gl + 2 * t < int(r.b.w) ? __ldg(A.nbr + r.b.z + gl + 2 * t) : -1;
-        u53 = draw_u53(seed, r.a.w, uint32_t(sweep), 0u);
+            nbr[t] = (ra.y >> 16) && gl < 2 && gl + 2 * t < int(rb.w) ? __ldg(A.nbr + rb.z + gl + 2 * t) : -1;
+        u53 = draw_u53(seed, ra.w, uint32_t(s0), 0u);
     };
     auto coef = [](const uint2& e) { return (e.x >> 31) ? -__uint_as_float(e.y) : __uint_as_float(e.y); };
-
-    // cur: the item in hand (its loads done or in flight); nx: the record after it
-    int pc = 0, pit = ip[0] + warp - kLocalWarps, psw = 0;
-    advance(pc, pit, psw);
-    Rec cur{}, nx{};
-    int c_at = pc, s_at = psw;
-    if (psw < A.sweeps) {
-        cur = rec_of(pit);
-        fetch(cur, psw);
-        advance(pc, pit, psw);
-        if (psw < A.sweeps) nx = rec_of(pit);
+    if (total > 0) {
+        settle();
+        na = __ldg(rec_of(it0));
+        nb = __ldg(rec_of(it0) + 1);
+        issue();
     }
+    // The barrier between a class and the next is joined by the warps that have
+    // items in either: those of the first only arrive, those of the second wait
+    // (named barriers 1 .. 15 in turn). A barrier's name comes round after 15
+    // classes: every class has an item, so with 15 warps a warp's next item lies
+    // at most 15 classes ahead, and when it comes to wait at the barrier before
+    // that class (at most 14 after the one it last joined), the last use of the
+    // name has completed. A refresh or a trace stops the whole CTA instead.
+    auto full_stop = [&](int sweep) {   // before the sweep's first class
+        return sweep > 0 && (A.trace != nullptr || (A.refresh > 0 && sweep % A.refresh == 0));
+    };
+    auto members = [&](int c) {   // threads of the barrier behind class c
+        const int d = c + 1 < nc ? c + 1 : 0;
+        return 32 * min(kLocalWarps, ip[c + 1] - ip[c] + ip[d + 1] - ip[d]);
+    };
+    auto wait_class = [&](int idx, int threads) {
+        __syncwarp();
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + idx % 15), "r"(threads) : "memory");
+    };
+    auto leave_class = [&](int idx, int threads) {
+        __syncwarp();
+        asm volatile("bar.arrive %0, %1;" ::"r"(1 + idx % 15), "r"(threads) : "memory");
+    };
+    bool ready = s0 == 0 && c0 == 0;   // nothing to wait for before the item in hand
     unsigned long long my_accepts = 0;
     for (int sweep = 0; sweep < A.sweeps; ++sweep) {
-        if (A.refresh > 0 && sweep > 0 && sweep % A.refresh == 0) {
-            // fp64 refresh, a thread per ray: rho = sum a' over its set bits in
-            // order - sqrt|w| d, the drift |hi + lo - rho| recorded
-            float dmax = 0.0f;
-            for (int b = tid; b < nr; b += kLocalThreads) {
-                const double sw = sqrt(fabs(A.w64[b]));
-                double acc = 0.0;
-                const int k1 = A.rrow[b + 1];
-                for (int k = A.rrow[b]; k < k1; ++k)
-                    if (bit_of(__ldg(A.rbit + k))) acc = __dadd_rn(acc, double(scaled_coef(sw, __ldg(A.ra + k))));
-                const double v = __dsub_rn(acc, __dmul_rn(sw, A.d[b]));
-                const float2 r = rho[b];
-                dmax = fmaxf(dmax, __double2float_rn(fabs(__dsub_rn(__dadd_rn(double(r.x), double(r.y)), v))));
-                rho[b] = split_pair(v);
+        if (full_stop(sweep)) {
+            __syncthreads();
+            if (A.trace && tid == 0) {   // the sweep before
+                A.trace[size_t(branch) * A.sweeps + sweep - 1] = s_trace;
+                s_trace = 0.0;
             }
-            if (dmax > 0.0f) atomicMax(reinterpret_cast<int*>(&A.drift[branch]), __float_as_int(dmax));
+            if (A.refresh > 0 && sweep % A.refresh == 0) {
+                // fp64 refresh, a thread per ray: rho = sum a' over its set bits in
+                // order - sqrt|w| d, the drift |hi + lo - rho| recorded
+                float dmax = 0.0f;
+                for (int b = tid; b < nr; b += kLocalThreads) {
+                    const double sw = sqrt(fabs(A.w64[b]));
+                    double acc = 0.0;
+                    const int k1 = A.rrow[b + 1];
+                    for (int k = A.rrow[b]; k < k1; ++k)
+                        if (bit_of(__ldg(A.rbit + k))) acc = __dadd_rn(acc, double(scaled_coef(sw, __ldg(A.ra + k))));
+                    const double v = __dsub_rn(acc, __dmul_rn(sw, A.d[b]));
+                    const float2 r = rho[b];
+                    dmax = fmaxf(dmax, __double2float_rn(fabs(__dsub_rn(__dadd_rn(double(r.x), double(r.y)), v))));
+                    rho[b] = split_pair(v);
+                }
+                if (dmax > 0.0f) atomicMax(reinterpret_cast<int*>(&A.drift[branch]), __float_as_int(dmax));
+            }
             __syncthreads();
         }
         const double T = A.temp[sweep];
         const float inv_T = float(1.0 / T);
-        for (int c = 0; c < nc; ++c) {
-            while (s_at == sweep && c_at == c) {   // the warp's items of this class
-                const uint32_t tag = cur.a.y;
-                const int nsg = int(tag >> 16), base = 2 * int((tag >> 5) & 31u), len = int(tag & 31u);
-                const int i = int(cur.a.z);
-                // the residuals of the lane's entries
+        while (s0 == sweep && total > 0) {
+            const int c = c0, idx = sweep * nc + c;
+            if (!ready && !(c == 0 && full_stop(sweep))) wait_class(idx - 1, members(c > 0 ? c - 1 : nc - 1));
+            do {   // the warp's items of this class
+                const uint32_t tag = ra.y;
+                const int nsg = int(tag >> 16), base = 2 * int((tag >> 5) & 31u);
+                const int i = int(ra.z);
                 float2 held[kHold];
 #pragma unroll
-                for (int u = 0; u < kHold; ++u) held[u] = rho[ent[u].x & kRay];   // entry 0 where there is none
-                const uint32_t xi = nsg ? bit_of(i) : 0u;
+                for (int u = 0; u < kHold; ++u) held[u] = rho[en[u].x & kRay];
+                const uint32_t xi = bit_of(i);
                 int unlike = 0;
 #pragma unroll
                 for (int t = 0; t < kNbrLane; ++t)
-                    if (nb[t] >= 0) unlike += int(bit_of(nb[t]) ^ xi);
+                    if (nbr[t] >= 0) unlike += int(bit_of(nbr[t]) ^ xi);
                 const int gl = lane - base;
                 if (nsg && gl < 2)
-                    for (int j = gl + 2 * kNbrLane; j < int(cur.b.w); j += 2) unlike += int(bit_of(__ldg(A.nbr + cur.b.z + j)) ^ xi);
+                    for (int j = gl + 2 * kNbrLane; j < int(rb.w); j += 2) unlike += int(bit_of(__ldg(A.nbr + rb.z + j)) ^ xi);
                 float acc = 0.0f;
 #pragma unroll
-                for (int u = 0; u < kHold; ++u)
-                    if (half + 2 * u < len) acc = fmaf(coef(ent[u]), __fadd_rn(held[u].x, held[u].y), acc);
+                for (int u = 0; u < kHold; ++u) acc = fmaf(coef(en[u]), __fadd_rn(held[u].x, held[u].y), acc);
                 const float seg = __fadd_rn(acc, __shfl_xor_sync(kAllLanes, acc, 1));
                 unlike += __shfl_xor_sync(kAllLanes, unlike, 1);
                 unlike = __shfl_sync(kAllLanes, unlike, base);
                 // the bit's segment sums in order
                 const int most = int(__reduce_max_sync(kAllLanes, unsigned(nsg)));
                 float h = 0.0f;
-                for (int q = 0; q < min(most, kPairs); ++q) {
-                    const float v = __shfl_sync(kAllLanes, seg, (base + 2 * q) & 31);
-                    if (q < nsg) h = __fadd_rn(h, v);
+                for (int q0 = 0; q0 < min(most, kPairs); q0 += 4) {
+                    float v[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) v[q] = __shfl_sync(kAllLanes, seg, (base + 2 * (q0 + q)) & 31);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        if (q0 + q < min(nsg, kPairs)) h = __fadd_rn(h, v[q]);
                 }
                 // a bit of more segments has the warp to itself: further rounds
                 auto last_of = [&](int q) { return q == nsg - 1 ? int((tag >> 10) & 31u) : q < nsg ? kSegE : 0; };
                 for (int r = kPairs; r < most; r += kPairs) {
-                    const int first = int(cur.a.x) + r * kSegE, l2 = last_of(r + pair);
+                    const int first = int(ra.x) + r * kSegE, l2 = last_of(r + pair);
                     float a2 = 0.0f;
                     for (int e = half; e < l2; e += 2) {
                         const uint2 en = __ldg(A.ent + first + e);
@@ -223,21 +261,20 @@ __global__ void __launch_bounds__(kLocalThreads, 1) resid_local_kernel(ResidLoca
                     for (int q = 0; q < min(most - r, kPairs); ++q) h = __fadd_rn(h, __shfl_sync(kAllLanes, s2, 2 * q));
                 }
                 const float delta = xi ? -1.0f : 1.0f;
-                const float t = __fadd_rn(__uint_as_float(cur.b.x), h);
-                const float prior = __fmul_rn(A.lambda, float(int(cur.b.w) - 2 * unlike));
-                const float dE = __fadd_rn(__fadd_rn(__fmul_rn(delta, t), __uint_as_float(cur.b.y)), prior);
+                const float t = __fadd_rn(__uint_as_float(rb.x), h);
+                const float prior = __fmul_rn(A.lambda, float(int(rb.w) - 2 * unlike));
+                const float dE = __fadd_rn(__fadd_rn(__fmul_rn(delta, t), __uint_as_float(rb.y)), prior);
                 const bool flip = nsg && (dE <= 0.0f || uphill_accept(u53, double(dE), T, inv_T));
                 if (flip) {
 #pragma unroll
-                    for (int u = 0; u < kHold; ++u)
-                        if (half + 2 * u < len)
-                            rho[ent[u].x & kRay] = two_sum_add(held[u], __fmul_rn(delta, __uint_as_float(ent[u].y)));
+                    for (int u = 0; u < kHold; ++u)   // rho += delta a'
+                        rho[en[u].x & kRay] = two_sum_add(held[u], __fmul_rn(delta, __uint_as_float(en[u].y)));
                     for (int r = kPairs; r < nsg; r += kPairs) {
-                        const int first = int(cur.a.x) + r * kSegE, l2 = last_of(r + pair);
+                        const int first = int(ra.x) + r * kSegE, l2 = last_of(r + pair);
                         for (int e = half; e < l2; e += 2) {
                             const uint2 en = __ldg(A.ent + first + e);
-                            float2& at = rho[en.x & kRay];
-                            at = two_sum_add(at, __fmul_rn(delta, __uint_as_float(en.y)));
+                            float2& to = rho[en.x & kRay];
+                            to = two_sum_add(to, __fmul_rn(delta, __uint_as_float(en.y)));
                         }
                     }
                     if (gl == 0) {
@@ -246,26 +283,24 @@ __global__ void __launch_bounds__(kLocalThreads, 1) resid_local_kernel(ResidLoca
                         if (A.trace) atomicAdd(&s_trace, double(dE));
                     }
                 }
-                // on to the next item: its record is here, its loads start
-                cur = nx;
-                c_at = pc;
-                s_at = psw;
-                if (psw < A.sweeps) {
-                    fetch(cur, psw);
-                    advance(pc, pit, psw);
-                    if (psw < A.sweeps) nx = rec_of(pit);
-                }
+                it0 += kLocalWarps;
+                settle();
+                if (s0 < A.sweeps) issue();
+            } while (s0 == sweep && c0 == c);
+            const bool last = c == nc - 1;
+            if (last && (sweep + 1 == A.sweeps || full_stop(sweep + 1))) {
+                ready = false;   // the whole CTA stops before the next class
+            } else if (last ? s0 == sweep + 1 && c0 == 0 : s0 == sweep && c0 == c + 1) {
+                wait_class(idx, members(c));
+                ready = true;
+            } else {
+                leave_class(idx, members(c));
+                ready = false;
             }
-            __syncthreads();
-        }
-        if (A.trace) {
-            if (tid == 0) {
-                A.trace[size_t(branch) * A.sweeps + sweep] = s_trace;
-                s_trace = 0.0;
-            }
-            __syncthreads();
         }
     }
+    __syncthreads();
+    if (A.trace && tid == 0) A.trace[size_t(branch) * A.sweeps + A.sweeps - 1] = s_trace;
     for (int i = tid; i < n; i += kLocalThreads) A.x_out[size_t(branch) * size_t(n) + size_t(A.order[i])] = uint8_t(bit_of(i));
     if (my_accepts) atomicAdd(&s_accepts, my_accepts);
     __syncthreads();
@@ -273,7 +308,7 @@ __global__ void __launch_bounds__(kLocalThreads, 1) resid_local_kernel(ResidLoca
 }
 
 size_t local_smem(int n, int n_rays, int n_colours) {
-    return size_t(n_rays) * 8 + size_t((n + 31) / 32) * 4 + (size_t(n_colours) + 1) * 4;
+    return (size_t(n_rays) + 1) * 8 + size_t((n + 31) / 32) * 4 + (size_t(n_colours) + 1) * 4;
 }
 
 }  // namespace
@@ -335,11 +370,26 @@ void resid_local_plan(ResidualPlan& P) {
     }
 }
 
-bool resid_local_route(const ResidualPlan& p) {
-    if (!p.local) return false;
+// Microseconds per sweep, fitted to B200 times at 500 to 90,000 bits: a class
+// step of the local sweep costs 1.05 or, once its items outnumber the warps,
+// 0.1 per item; the lockstep sweep 3.9 per class at 16 branches and 13 % more
+// per further 16 (90,000 bits: 16 branches 1.09 ms local, 0.88 lockstep; 64
+// branches 1.09 and 1.22; 40,000 bits, 64 branches 0.54 and 0.83).
+bool resid_local_route(const ResidualPlan& p, int R) {
+    if (!p.local || std::getenv("QB_PHASE_TIMES") || std::getenv("QB_TEST_BARRIER_STALL")) return false;
     const char* k = std::getenv("QB_RESID_KERNEL");
-    return !(k && std::strcmp(k, "lockstep") == 0) && !std::getenv("QB_PHASE_TIMES") &&
-           !std::getenv("QB_TEST_BARRIER_STALL");
+    if (k && std::strcmp(k, "lockstep") == 0) return false;
+    if (k && std::strcmp(k, "local") == 0) return true;
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const double classes = p.col.n_colours(), items = p.l_ptr.empty() ? 0.0 : p.l_ptr.back();
+    const double local = std::max(1.05 * classes, 0.1 * items) * ((R + sms - 1) / sms);
+    double lock = 0.0;
+    for (int left = R; left > 0; left -= resid_lockstep_max_branches()) {
+        const int groups = (std::min(left, resid_lockstep_max_branches()) + 15) / 16;
+        lock += 3.9 * classes * (1.0 + 0.13 * (groups - 1));
+    }
+    return local < lock;
 }
 
 qb_status launch_resid_local(const ResidualPlan& p, const SolveBuffers& b, int R, int sweeps, int refresh, uint64_t seed0,

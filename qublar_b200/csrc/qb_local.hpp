@@ -14,10 +14,11 @@ bool resid_local_fit(int n, int n_rays, int n_colours);
 // The work table of the local sweep (host): per class, warp items of 16 lane
 // pairs, a pair per 16-entry segment, a bit's pairs side by side.
 void resid_local_plan(ResidualPlan& P);
-// Whether a solve takes the local sweep: a plan that has it, unless the
-// lockstep kernel is asked for (QB_RESID_KERNEL=lockstep, its phase times, or
-// its barrier's test hook).
-bool resid_local_route(const ResidualPlan& p);
+// Whether a solve of R branches takes the local sweep: a plan that has it and
+// whose estimated sweep time is the shorter one, unless the lockstep kernel is
+// asked for (QB_RESID_KERNEL=lockstep, its phase times, or its barrier's test
+// hook; QB_RESID_KERNEL=local asks for the local one).
+bool resid_local_route(const ResidualPlan& p, int R);
 // Branches seed0 .. seed0 + R - 1; the buffers of launch_resid_lockstep (no scratch).
 qb_status launch_resid_local(const ResidualPlan& p, const SolveBuffers& b, int R, int sweeps, int refresh, uint64_t seed0,
                              cudaStream_t st);

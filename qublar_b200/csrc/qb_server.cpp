@@ -350,7 +350,7 @@ qb_status launch_coop(qb_server* S, Request* r, cudaStream_t st, int qubo_ctas) 
         if ((s = launch_qubo_energies(r->prob->qubo, x, r->R, r->d_ef64.as<double>(), st))) return s;
     } else {
         const ResidualPlan& P = r->prob->resid;
-        const bool local = resid_local_route(P);
+        const bool local = resid_local_route(P, r->R);
         const int RB = local ? r->R : resid_lockstep_max_branches();
         for (int b0 = 0; b0 < r->R; b0 += RB) {
             SolveBuffers b;

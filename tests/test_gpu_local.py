@@ -50,7 +50,10 @@ def test_equals_the_lockstep_sweep_and_the_oracle(name, monkeypatch):
     arr = make()
     P = ResidualProblem.from_arrays(arr)
     s = Schedule(20.0, 0.6, sweeps, 6, 11)
+    monkeypatch.setenv("QB_RESID_KERNEL", "local")
     r = P.solve(s, R, 3, trace=True)
+    u = P.solve(s, R, 3)   # without the trace: class barriers across sweeps too
+    assert (u.branches() == r.branches()).all()
     monkeypatch.setenv("QB_RESID_KERNEL", "lockstep")
     o = P.solve(s, R, 3, trace=True)
     monkeypatch.delenv("QB_RESID_KERNEL")
