@@ -1334,14 +1334,15 @@ extern "C" qb_status qb_solve(qb_problem* p, const qb_schedule* sch, uint32_t n_
             if ((s = alloc_async(r->d_drift, size_t(R) * sizeof(float), st))) return bail(s);
             if ((s = alloc_async(r->d_accepts, size_t(R) * 8, st))) return bail(s);
             if ((s = alloc_async(r->d_e_track, size_t(R) * 8, st))) return bail(s);
-            if ((s = alloc_async(r->d_scratch, qubo_scratch(P), st))) return bail(s);
+            const bool small = qubo_small_fit(P);
+            if (!small && (s = alloc_async(r->d_scratch, qubo_scratch(P), st))) return bail(s);
             if (cudaMemsetAsync(r->d_drift.p, 0, size_t(R) * sizeof(float), st) != cudaSuccess ||
                 cudaMemsetAsync(r->d_accepts.p, 0, size_t(R) * 8, st) != cudaSuccess ||
                 cudaMemsetAsync(r->d_e_track.p, 0, size_t(R) * 8, st) != cudaSuccess ||
-                cudaMemsetAsync(r->d_scratch.p, 0, 64, st) != cudaSuccess)
+                (!small && cudaMemsetAsync(r->d_scratch.p, 0, 64, st) != cudaSuccess))
                 return bail(cuda_fail(cudaGetLastError(), "cudaMemsetAsync", __FILE__, __LINE__));
-            r->d_err = reinterpret_cast<const int*>(static_cast<const char*>(r->d_scratch.p) + 16);
-            const int RB = qubo_max_branches();
+            if (!small) r->d_err = reinterpret_cast<const int*>(static_cast<const char*>(r->d_scratch.p) + 16);
+            const int RB = small ? R : qubo_max_branches();
             cudaEventRecord(r->ev0, st);
             int anneal_launches = 0;
             for (int b0 = 0; b0 < R && s == QB_OK; b0 += RB, ++anneal_launches) {
@@ -1353,8 +1354,9 @@ extern "C" qb_status qb_solve(qb_problem* p, const qb_schedule* sch, uint32_t n_
                 qbuf.accepts = r->d_accepts.as<unsigned long long>() + b0;
                 qbuf.trace = b.trace ? b.trace + size_t(b0) * size_t(r->sweeps) : nullptr;
                 qbuf.scratch = r->d_scratch.p;
-                s = launch_qubo_lockstep(P, qbuf, std::min(RB, R - b0), r->sweeps, sch->refresh_sweeps,
-                                         seed0 + uint64_t(b0), st);
+                s = small ? launch_qubo_small(P, qbuf, R, r->sweeps, sch->refresh_sweeps, seed0, st)
+                          : launch_qubo_lockstep(P, qbuf, std::min(RB, R - b0), r->sweeps, sch->refresh_sweeps,
+                                                 seed0 + uint64_t(b0), st);
             }
             if (s != QB_OK) return bail(s);
             cudaEventRecord(r->ev1, st);

@@ -30,6 +30,11 @@ size_t qubo_scratch(const QuboPlan& p);
 // of the device to other work; the branches do not depend on it).
 qb_status launch_qubo_lockstep(const QuboPlan& p, const QuboBuffers& b, int R, int sweeps, int refresh, uint64_t seed0,
                                cudaStream_t st, int ctas = 0);
+// A problem whose fields of 32 replicas fit one CTA's shared memory
+// (qb_qubo_local.cu): any R in one launch, a CTA per 32 replicas; no scratch.
+bool qubo_small_fit(const QuboPlan& p);
+qb_status launch_qubo_small(const QuboPlan& p, const QuboBuffers& b, int R, int sweeps, int refresh, uint64_t seed0,
+                            cudaStream_t st);
 qb_status launch_qubo_energies(const QuboPlan& p, const uint8_t* x, int K, double* e, cudaStream_t st);
 
 }  // namespace qb

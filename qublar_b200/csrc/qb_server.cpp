@@ -334,7 +334,8 @@ qb_status launch_coop(qb_server* S, Request* r, cudaStream_t st, int qubo_ctas) 
     }
     uint8_t* x = r->d_x.as<uint8_t>();
     if (qubo) {
-        const int RB = qubo_max_branches();
+        const bool small = qubo_small_fit(r->prob->qubo);
+        const int RB = small ? r->R : qubo_max_branches();
         for (int b0 = 0; b0 < r->R; b0 += RB) {
             QuboBuffers qb;
             qb.x = x + size_t(b0) * size_t(r->n);
@@ -343,9 +344,10 @@ qb_status launch_coop(qb_server* S, Request* r, cudaStream_t st, int qubo_ctas) 
             qb.e_track = r->d_etrack.as<double>() + b0;
             qb.accepts = r->d_accepts.as<unsigned long long>() + b0;
             qb.scratch = r->d_state.p;
-            if ((s = launch_qubo_lockstep(r->prob->qubo, qb, std::min(RB, r->R - b0), r->sweeps,
-                                          r->sched.refresh_sweeps, r->seed0 + uint64_t(b0), st, qubo_ctas)))
-                return s;
+            s = small ? launch_qubo_small(r->prob->qubo, qb, r->R, r->sweeps, r->sched.refresh_sweeps, r->seed0, st)
+                      : launch_qubo_lockstep(r->prob->qubo, qb, std::min(RB, r->R - b0), r->sweeps,
+                                             r->sched.refresh_sweeps, r->seed0 + uint64_t(b0), st, qubo_ctas);
+            if (s != QB_OK) return s;
         }
         if ((s = launch_qubo_energies(r->prob->qubo, x, r->R, r->d_ef64.as<double>(), st))) return s;
     } else {
