@@ -28,6 +28,7 @@
 #include "qb_kernels.hpp"
 #include "qb_local.hpp"
 #include "qb_qubo.hpp"
+#include "qb_word.hpp"
 
 using namespace qb;
 
@@ -87,6 +88,7 @@ struct Request {
     DevBuf d_x, d_f, d_e, d_p, d_temp, d_state, d_drift, d_accepts, d_ef64, d_etrack;
     // ising progress
     std::vector<Group> groups;
+    int np = 0;           // word units of 2 np replicas (0: groups of the field-carrying kernel)
     int cursor = 0;       // next sweep
     int slice = 1;        // sweeps per tick
     // residual
@@ -117,6 +119,10 @@ struct qb_server {
     int next_resid_stream = 0;
     cudaEvent_t upload_ev = nullptr, tick_ev = nullptr;
     BatchShape shape;
+    bool smem_asked = false;   // the caller bounded an ising item's shared-memory state
+    DevBuf d_words;            // the tick's word units: counters, items, bundles
+    unsigned char* h_words = nullptr;
+    size_t words_cap = 0;
     DevBuf d_tick;
     unsigned char* h_tick = nullptr;
     size_t tick_cap = 0;   // items the tick buffers hold
@@ -231,6 +237,32 @@ void plan_groups(qb_server* S, Request* r, double target_attempts) {
     r->slice = int(std::max(1.0, std::min(double(r->sweeps), std::floor(target_attempts / per_sweep))));
 }
 
+// Whether an ising request runs as word units (qb_word.cu): one coupling size,
+// at least four replicas, words that fit a CTA; not where the caller's bound on
+// an item's state asks for global state.
+bool as_words(const qb_server* S, const Request* r) {
+    const IsingPlan& P = r->prob->ising;
+    return word_sweep(P) && r->R >= 4 && word_item_smem(P, 2) <= word_max_smem() &&
+           !(S->smem_asked && batch_item_smem(r->n, 1) > size_t(S->shape.smem_bytes));
+}
+
+// Bytes of a word unit's kept state.
+size_t word_state_bytes(int n, int np) { return (size_t(n) * size_t(np > 4 ? np / 4 : 1) + 255) / 256 * 256; }
+
+// Narrow units while a unit's average class still fills a CTA (the request
+// spreads over more SMs), and slices that last about the tick target on one SM
+// (two instructions a cycle and SM scheduler pair, 1.9 GHz).
+void plan_words(qb_server* S, Request* r) {
+    const IsingPlan& P = r->prob->ising;
+    int np = 16;
+    while (np > 2 && (np >= r->R || word_item_smem(P, np) > word_max_smem() ||
+                      word_class_passes(P.n, P.col.n_colours(), np / 2) >= kWordThreads / 32))
+        np /= 2;
+    r->np = np;
+    const double us = word_unit_cost(P.n, P.nnz, np, 1) / 3800.0;
+    r->slice = int(std::max(1.0, std::min(double(r->sweeps), std::floor(double(S->cfg.tick_target_us) / us))));
+}
+
 // The grid of a cooperative request that runs beside others: enough CTAs
 // that a colour class gives each of them about one round of warp items (a
 // residual bit takes about nnz / (16 n) + 1.5 items, a QUBO bit one warp
@@ -260,9 +292,14 @@ qb_status admit_ising(qb_server* S, Request* r) {
     const std::vector<double> temp = temperatures(r->sched);
     if ((s = upload_vec(r->d_temp, temp, S->upload_stream))) return s;
     double target = double(S->cfg.tick_target_us) * 1e-6 * 4e8;   // attempts one CTA does in the target time
-    plan_groups(S, r, target);
     int64_t state = 0;
-    for (const Group& g : r->groups) state += int64_t(batch_item_smem(r->n, g.G) + 255) / 256 * 256;
+    if (as_words(S, r)) {
+        plan_words(S, r);
+        state = int64_t(word_state_bytes(r->n, r->np)) * ((r->R + 2 * r->np - 1) / (2 * r->np));
+    } else {
+        plan_groups(S, r, target);
+        for (const Group& g : r->groups) state += int64_t(batch_item_smem(r->n, g.G) + 255) / 256 * 256;
+    }
     if ((s = r->d_state.alloc(size_t(state)))) return s;
     if ((s = r->d_x.alloc(size_t(r->R) * size_t(r->n)))) return s;
     if ((s = r->d_f.alloc(size_t(r->R) * size_t(r->n) * 4))) return s;
@@ -298,7 +335,9 @@ qb_status launch_resid(qb_server* S, Request* r) {
     b.accepts = r->d_accepts.as<unsigned long long>();
     b.e_f64 = r->d_ef64.as<double>();
     b.p = r->d_p.as<float>();
-    if ((s = launch_resid_anneal(P, b, r->R, r->sweeps, r->sched.refresh_sweeps, r->seed0, st))) return s;
+    if (resid_local_route(P, r->R)) s = launch_resid_local(P, b, r->R, r->sweeps, r->sched.refresh_sweeps, r->seed0, st);
+    else s = launch_resid_anneal(P, b, r->R, r->sweeps, r->sched.refresh_sweeps, r->seed0, st);
+    if (s != QB_OK) return s;
     if ((s = launch_resid_energies(P, b.x, r->R, b.e_f64, st))) return s;
     if ((s = launch_marginals(b.x, r->R, r->n, b.p, st))) return s;
     QB_CUDA(cudaEventCreateWithFlags(&r->done_ev, cudaEventDisableTiming));
@@ -498,13 +537,77 @@ qb_status ensure_tick_capacity(qb_server* S, size_t items) {
     return QB_OK;
 }
 
+// The tick's word units: their tables up from pinned memory and the launch.
+qb_status launch_word_units(qb_server* S, std::vector<WordUnit>& units) {
+    const WordWork w = word_pack(units);
+    constexpr size_t kCtl = 256;
+    const size_t ib = w.items.size() * sizeof(WordItem), bb = w.bundles.size() * sizeof(WordBundle);
+    if (kCtl + ib + bb > S->words_cap) {
+        size_t cap = std::max<size_t>(1 << 16, S->words_cap);
+        while (cap < kCtl + ib + bb) cap *= 2;
+        QB_CUDA(cudaStreamSynchronize(S->tick_stream));
+        if (S->h_words) cudaFreeHost(S->h_words);
+        S->h_words = nullptr;
+        S->words_cap = 0;
+        QB_CUDA(cudaMallocHost(&S->h_words, cap));
+        qb_status s = S->d_words.alloc(cap);
+        if (s != QB_OK) return s;
+        S->words_cap = cap;
+    }
+    std::memcpy(S->h_words + kCtl, w.items.data(), ib);
+    std::memcpy(S->h_words + kCtl + ib, w.bundles.data(), bb);
+    unsigned char* d = S->d_words.as<unsigned char>();
+    QB_CUDA(cudaMemcpyAsync(d + kCtl, S->h_words + kCtl, ib + bb, cudaMemcpyHostToDevice, S->tick_stream));
+    return launch_ising_words(w, reinterpret_cast<const WordItem*>(d + kCtl),
+                              reinterpret_cast<const WordBundle*>(d + kCtl + ib), reinterpret_cast<int*>(d), S->tick_stream);
+}
+
+// The tick's items of the field-carrying kernel: one graph replay (or copy and launch).
+qb_status launch_items(qb_server* S, const std::vector<IsingItem>& items) {
+    qb_status s;
+    int* ctl = reinterpret_cast<int*>(S->h_tick);
+    ctl[0] = 0;
+    ctl[1] = int(items.size());
+    std::memcpy(S->h_tick + kTickHeader, items.data(), items.size() * sizeof(IsingItem));
+    const size_t bytes = kTickHeader + items.size() * sizeof(IsingItem);
+    if (S->cfg.use_graph) {
+        QB_CUDA(cudaGraphExecMemcpyNodeSetParams1D(S->exec, S->copy_node, S->d_tick.p, S->h_tick, bytes,
+                                                   cudaMemcpyHostToDevice));
+        QB_CUDA(cudaGraphLaunch(S->exec, S->tick_stream));
+    } else {
+        QB_CUDA(cudaMemcpyAsync(S->d_tick.p, S->h_tick, bytes, cudaMemcpyHostToDevice, S->tick_stream));
+        if ((s = launch_ising_batch_ctl(reinterpret_cast<const IsingItem*>(S->d_tick.as<unsigned char>() + kTickHeader),
+                                        S->d_tick.as<int>(), S->shape, S->tick_stream)))
+            return s;
+    }
+    return QB_OK;
+}
+
 qb_status launch_tick(qb_server* S) {
     std::vector<IsingItem> items;
+    std::vector<WordUnit> units;
     S->tick_members.clear();
     for (Request* r : S->running_ising) {
         if (r->cancel) continue;
         const IsingPlan& P = r->prob->ising;
         const int s0 = r->cursor, s1 = std::min(r->sweeps, r->cursor + r->slice);
+        for (int q = 0; r->np > 0 && 2 * q * r->np < r->R; ++q) {
+            const int r0 = 2 * q * r->np;
+            WordUnit u;
+            word_fill(u.item, P, r->np, std::min(2 * r->np, r->R - r0), r->seed0 + uint64_t(r0));
+            u.item.temp = r->d_temp.as<double>();
+            u.item.state = r->d_state.as<unsigned char>() + size_t(q) * word_state_bytes(r->n, r->np);
+            u.item.sweep0 = s0;
+            u.item.sweep1 = s1;
+            u.item.flags = (s0 == 0 ? kItemInit : 0) | (s1 == r->sweeps ? kItemFinal : kItemKeep);
+            u.item.e_out = r->d_e.as<long long>() + r0;
+            u.item.x_out = r->d_x.as<uint8_t>() + size_t(r0) * size_t(r->n);
+            u.item.f_out = r->d_f.as<int32_t>() + size_t(r0) * size_t(r->n);
+            u.smem = word_item_smem(P, r->np);
+            u.cost = word_unit_cost(P.n, P.nnz, r->np, s1 - s0);
+            u.passes = word_class_passes(P.n, P.col.n_colours(), r->np);
+            units.push_back(u);
+        }
         for (const Group& g : r->groups) {
             IsingItem it;
             std::memset(&it, 0, sizeof(it));
@@ -535,31 +638,18 @@ qb_status launch_tick(qb_server* S) {
         }
         S->tick_members.emplace_back(r, s1);
     }
-    if (items.empty()) return QB_OK;
+    if (items.empty() && units.empty()) return QB_OK;
     // largest first, as in a batch
     std::stable_sort(items.begin(), items.end(), [](const IsingItem& a, const IsingItem& b) {
         return double(a.n) * (1 << a.log2g) * (a.sweep1 - a.sweep0) > double(b.n) * (1 << b.log2g) * (b.sweep1 - b.sweep0);
     });
-    qb_status s = ensure_tick_capacity(S, items.size());
+    qb_status s = items.empty() ? QB_OK : ensure_tick_capacity(S, items.size());
     if (s != QB_OK) return s;
     // the uploads of newly admitted requests come first
     QB_CUDA(cudaEventRecord(S->upload_ev, S->upload_stream));
     QB_CUDA(cudaStreamWaitEvent(S->tick_stream, S->upload_ev, 0));
-    int* ctl = reinterpret_cast<int*>(S->h_tick);
-    ctl[0] = 0;
-    ctl[1] = int(items.size());
-    std::memcpy(S->h_tick + kTickHeader, items.data(), items.size() * sizeof(IsingItem));
-    const size_t bytes = kTickHeader + items.size() * sizeof(IsingItem);
-    if (S->cfg.use_graph) {
-        QB_CUDA(cudaGraphExecMemcpyNodeSetParams1D(S->exec, S->copy_node, S->d_tick.p, S->h_tick, bytes,
-                                                   cudaMemcpyHostToDevice));
-        QB_CUDA(cudaGraphLaunch(S->exec, S->tick_stream));
-    } else {
-        QB_CUDA(cudaMemcpyAsync(S->d_tick.p, S->h_tick, bytes, cudaMemcpyHostToDevice, S->tick_stream));
-        if ((s = launch_ising_batch_ctl(reinterpret_cast<const IsingItem*>(S->d_tick.as<unsigned char>() + kTickHeader),
-                                        S->d_tick.as<int>(), S->shape, S->tick_stream)))
-            return s;
-    }
+    if (!units.empty() && (s = launch_word_units(S, units)) != QB_OK) return s;
+    if (!items.empty() && (s = launch_items(S, items)) != QB_OK) return s;
     for (auto& m : S->tick_members)
         if (m.second == m.first->sweeps) {
             Request* r = m.first;
@@ -569,7 +659,6 @@ qb_status launch_tick(qb_server* S) {
     S->tick_inflight = true;
     return QB_OK;
 }
-
 void fail_all_running(qb_server* S, qb_status st, const std::string& msg) {
     std::vector<Request*> all(S->running_ising);
     all.insert(all.end(), S->running_resid.begin(), S->running_resid.end());
@@ -787,6 +876,7 @@ extern "C" qb_status qb_server_create(const qb_server_config* cfg, qb_server** o
         const int cap = batch_max_smem();
         if (cap <= 0) return fail(QB_ECUDA, "qb_server_create: cannot read the shared-memory limit");
         c.batch.smem_bytes = std::min(c.batch.smem_bytes, cap);
+        S->smem_asked = cfg && cfg->batch.smem_bytes != 0;
         S->cfg = c;
         S->shape.threads = c.batch.threads;
         S->shape.smem_bytes = c.batch.smem_bytes;
@@ -1055,6 +1145,7 @@ extern "C" void qb_server_destroy(qb_server* S) {
     if (S->exec) cudaGraphExecDestroy(S->exec);
     if (S->graph) cudaGraphDestroy(S->graph);
     if (S->tick_stream) cudaStreamSynchronize(S->tick_stream);
+    if (S->h_words) cudaFreeHost(S->h_words);
     if (S->h_tick) cudaFreeHost(S->h_tick);
     S->d_tick.release();
     for (cudaStream_t st : S->resid_streams) {
