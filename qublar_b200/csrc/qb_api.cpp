@@ -718,7 +718,7 @@ qb_status plan_residual(const qb_residual_desc* d, ResidualPlan& P, int lock_sli
         P.chunk_ptr[size_t(t) + 1] = int32_t(P.chunks.size() / 8);
     }
     mark("chunks");
-    P.local = lock && resid_local_fit(n, nr, nc);
+    P.local = resid_local_fit(n, nr, nc);
     if (P.local) {
         resid_local_plan(P);
         mark("local items");
@@ -739,6 +739,7 @@ int64_t residual_device_bytes(const ResidualPlan& P) {
                         P.chunk_ptr.size()) * 4;
     b += (nr + 1) * 4 + nnz * 12 + n * 8 + nr * 16 + (n + 1) * 4 + P.n_nbr * 4;   // ray-major CSR (two bit orders)
     if (P.local) b += int64_t(P.l_rec.size() + P.l_ptr.size()) * 4;
+    if (P.local && P.variant != QB_RESID_LOCKSTEP) b += int64_t(P.h_nbr_new.size()) * 4 + nnz * 4;
     if (P.variant == QB_RESID_LOCKSTEP) b += int64_t(P.h_meta.size() + P.h_nbr_new.size()) * 4 + nnz * 4;
     return b;
 }
@@ -844,7 +845,8 @@ qb_status upload_residual(ResidualPlan& P, const qb_residual_desc* d, cudaStream
         if ((s = P.d_o_rbit.alloc(size_t(P.nnz) * 4))) return s;
         if ((s = P.d_rbit.alloc(size_t(P.nnz) * 4))) return s;
         if ((s = P.d_ra.alloc(size_t(P.nnz) * 4))) return s;
-        DevBuf& rbn = lock ? P.d_rbit_new : t_rbit_n;   // sweep positions: kept by the lockstep sweep only
+        const bool keep_pos = lock || P.local;
+        DevBuf& rbn = keep_pos ? P.d_rbit_new : t_rbit_n;   // sweep positions: kept where a sweep's refresh reads them
         if ((s = rbn.alloc(size_t(P.nnz) * 4))) return s;
         if ((s = t_rcount.alloc(size_t(std::max(nr, 1)) * 4))) return s;
         if ((s = t_cursor.alloc(size_t(std::max(nr, 1)) * 4))) return s;
@@ -879,7 +881,7 @@ qb_status upload_residual(ResidualPlan& P, const qb_residual_desc* d, cudaStream
     if (!on_device) {
         QB_UP(d_ent, ent); QB_UP(d_row, P.h_row); QB_UP(d_order, C.order);
         QB_UP(d_rrow, rrow); QB_UP(d_rbit, rbit_h); QB_UP(d_ra, ra); QB_UP(d_o_rbit, rbit_o);
-        if (lock) QB_UP(d_rbit_new, rbit_n);
+        if (lock || P.local) QB_UP(d_rbit_new, rbit_n);
         if ((s = upload(P.d_w64, d->w, size_t(nr) * 8, st))) return s;
     }
     QB_UP(d_lin, P.h_lin); QB_UP(d_q, P.h_q);
@@ -891,6 +893,7 @@ qb_status upload_residual(ResidualPlan& P, const qb_residual_desc* d, cudaStream
     }
     if (P.local) {
         QB_UP(d_lrec, P.l_rec); QB_UP(d_lptr, P.l_ptr);
+        if (!lock) QB_UP(d_nbr_new, P.h_nbr_new);
     }
 #undef QB_UP
     if ((s = upload(P.d_d, d->d, size_t(nr) * 8, st))) return s;

@@ -81,10 +81,19 @@ struct ResidLocalArgs {
 // of its bit << 5 | length of the bit's last segment << 10 | the bit's segments
 // << 16 (0: empty pair); the bit's sweep position; its input index; lin, q,
 // first neighbour, neighbours.
+// The cluster order's record: first entry; rays | flags; the rest alike.
+constexpr uint32_t kHeavyTag = 1u << 16, kLiveTag = 1u << 17;
+constexpr int kGroupRecs = 4;
+constexpr int kHeavyRays = 64;
 __host__ __device__ inline uint32_t rec_tag(int len, int pair, int last, int segs) {
     return uint32_t(len) | uint32_t(pair) << 5 | uint32_t(last) << 10 | uint32_t(segs) << 16;
 }
 
+// GROUPS: the cluster sweep's order (qb_kernels.cu) instead: eight lanes per
+// bit, 32 for one of more than 64 rays, each the fmaf chain over every eighth
+// (32nd) entry, joined by an xor butterfly; an item is four bits or one heavy
+// bit, and a lane past its eight entries goes on with the same chain.
+template <bool GROUPS>
 __global__ void __launch_bounds__(kLocalThreads, 1) resid_local_kernel(ResidLocalArgs A) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ double s_trace;
@@ -95,7 +104,8 @@ __global__ void __launch_bounds__(kLocalThreads, 1) resid_local_kernel(ResidLoca
     int32_t* ip = reinterpret_cast<int32_t*>(xs + words);
     const int tid = int(threadIdx.x), lane = tid & 31;
     const int warp = __shfl_sync(kAllLanes, tid >> 5, 0);
-    const int pair = lane >> 1, half = lane & 1;
+    const int pair = GROUPS ? lane >> 3 : lane >> 1, half = lane & 1;
+    constexpr int kRecs = GROUPS ? kGroupRecs : kPairs;   // records per item
     const int branch = int(blockIdx.x);
     const uint64_t seed = A.seed0 + uint64_t(branch);
     for (int b = tid; b < nr; b += kLocalThreads) rho[b] = split_pair(-__dmul_rn(sqrt(fabs(A.w64[b])), A.d[b]));
@@ -122,7 +132,7 @@ __global__ void __launch_bounds__(kLocalThreads, 1) resid_local_kernel(ResidLoca
         }
         while (it0 >= ip[c0 + 1]) ++c0;
     };
-    auto rec_of = [&](int it) { return A.rec + (size_t(it) * kPairs + size_t(pair)) * 2; };
+    auto rec_of = [&](int it) { return A.rec + (size_t(it) * kRecs + size_t(pair)) * 2; };
     // The item in hand: its record, and per entry of the lane its residual and
     // coefficient; entries past the segment are the zero pair rho[nr] with a
     // zero coefficient, which change nothing. na, nb: the next item's record.
@@ -140,17 +150,29 @@ __global__ void __launch_bounds__(kLocalThreads, 1) resid_local_kernel(ResidLoca
         const uint4* next = rec_of(ni);
         na = __ldg(next);
         nb = __ldg(next + 1);
-        const int len = int(ra.y & 31u);
+        if constexpr (GROUPS) {
+            const int rays = int(ra.y & 0xFFFFu);
+            const bool heavy = (ra.y & kHeavyTag) != 0;
+            const int gl = heavy ? lane : lane & 7, G = heavy ? 32 : 8;
 #pragma unroll
-        for (int u = 0; u < kHold; ++u) {
-            en[u] = make_uint2(uint32_t(nr), 0u);
-            if (half + 2 * u < len) en[u] = __ldg(A.ent + ra.x + half + 2 * u);
+            for (int u = 0; u < kHold; ++u) {
+                en[u] = make_uint2(uint32_t(nr), 0u);
+                if (gl + G * u < rays) en[u] = __ldg(A.ent + ra.x + gl + G * u);
+            }
+            nbr[0] = gl < int(rb.w) && (ra.y & kLiveTag) ? __ldg(A.nbr + rb.z + gl) : -1;
+        } else {
+            const int len = int(ra.y & 31u);
+#pragma unroll
+            for (int u = 0; u < kHold; ++u) {
+                en[u] = make_uint2(uint32_t(nr), 0u);
+                if (half + 2 * u < len) en[u] = __ldg(A.ent + ra.x + half + 2 * u);
+            }
+            // lanes 0 and 1 of the bit share its neighbours
+            const int gl = lane - 2 * int((ra.y >> 5) & 31u);
+#pragma unroll
+            for (int t = 0; t < kNbrLane; ++t)
+                nbr[t] = (ra.y >> 16) && gl < 2 && gl + 2 * t < int(rb.w) ? __ldg(A.nbr + rb.z + gl + 2 * t) : -1;
         }
-        // lanes 0 and 1 of the bit share its neighbours
-        const int gl = lane - 2 * int((ra.y >> 5) & 31u);
-#pragma unroll
-        for (int t = 0; t < kNbrLane; ++t)
-            nbr[t] = (ra.y >> 16) && gl < 2 && gl + 2 * t < int(rb.w) ? __ldg(A.nbr + rb.z + gl + 2 * t) : -1;
         u53 = draw_u53(seed, ra.w, uint32_t(s0), 0u);
     };
     auto coef = [](const uint2& e) { return (e.x >> 31) ? -__uint_as_float(e.y) : __uint_as_float(e.y); };
@@ -216,71 +238,124 @@ __global__ void __launch_bounds__(kLocalThreads, 1) resid_local_kernel(ResidLoca
             const int c = c0, idx = sweep * nc + c;
             if (!ready && !(c == 0 && full_stop(sweep))) wait_class(idx - 1, members(c > 0 ? c - 1 : nc - 1));
             do {   // the warp's items of this class
-                const uint32_t tag = ra.y;
-                const int nsg = int(tag >> 16), base = 2 * int((tag >> 5) & 31u);
-                const int i = int(ra.z);
-                float2 held[kHold];
+                if constexpr (GROUPS) {
+                    const bool heavy = (ra.y & kHeavyTag) != 0, live = (ra.y & kLiveTag) != 0;   // heavy: warp-uniform
+                    const int gl = heavy ? lane : lane & 7, G = heavy ? 32 : 8;
+                    const int rays = int(ra.y & 0xFFFFu), i = int(ra.z);
+                    float2 held[kHold];
 #pragma unroll
-                for (int u = 0; u < kHold; ++u) held[u] = rho[en[u].x & kRay];
-                const uint32_t xi = bit_of(i);
-                int unlike = 0;
+                    for (int u = 0; u < kHold; ++u) held[u] = rho[en[u].x & kRay];
+                    const uint32_t xi = bit_of(i);
+                    int unlike = nbr[0] >= 0 ? int(bit_of(nbr[0]) ^ xi) : 0;
+                    if (live)
+                        for (int q = gl + G; q < int(rb.w); q += G) unlike += int(bit_of(__ldg(A.nbr + rb.z + q)) ^ xi);
+                    float acc = 0.0f;
 #pragma unroll
-                for (int t = 0; t < kNbrLane; ++t)
-                    if (nbr[t] >= 0) unlike += int(bit_of(nbr[t]) ^ xi);
-                const int gl = lane - base;
-                if (nsg && gl < 2)
-                    for (int j = gl + 2 * kNbrLane; j < int(rb.w); j += 2) unlike += int(bit_of(__ldg(A.nbr + rb.z + j)) ^ xi);
-                float acc = 0.0f;
-#pragma unroll
-                for (int u = 0; u < kHold; ++u) acc = fmaf(coef(en[u]), __fadd_rn(held[u].x, held[u].y), acc);
-                const float seg = __fadd_rn(acc, __shfl_xor_sync(kAllLanes, acc, 1));
-                unlike += __shfl_xor_sync(kAllLanes, unlike, 1);
-                unlike = __shfl_sync(kAllLanes, unlike, base);
-                // the bit's segment sums in order
-                const int most = int(__reduce_max_sync(kAllLanes, unsigned(nsg)));
-                float h = 0.0f;
-                for (int q0 = 0; q0 < min(most, kPairs); q0 += 4) {
-                    float v[4];
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) v[q] = __shfl_sync(kAllLanes, seg, (base + 2 * (q0 + q)) & 31);
-#pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        if (q0 + q < min(nsg, kPairs)) h = __fadd_rn(h, v[q]);
-                }
-                // a bit of more segments has the warp to itself: further rounds
-                auto last_of = [&](int q) { return q == nsg - 1 ? int((tag >> 10) & 31u) : q < nsg ? kSegE : 0; };
-                for (int r = kPairs; r < most; r += kPairs) {
-                    const int first = int(ra.x) + r * kSegE, l2 = last_of(r + pair);
-                    float a2 = 0.0f;
-                    for (int e = half; e < l2; e += 2) {
-                        const uint2 en = __ldg(A.ent + first + e);
-                        const float2 rv = rho[en.x & kRay];
-                        a2 = fmaf(coef(en), __fadd_rn(rv.x, rv.y), a2);
+                    for (int u = 0; u < kHold; ++u) acc = fmaf(coef(en[u]), __fadd_rn(held[u].x, held[u].y), acc);
+                    for (int e = gl + G * kHold; e < rays; e += G) {   // a heavy bit of more than 256 rays
+                        const uint2 x = __ldg(A.ent + ra.x + e);
+                        const float2 rv = rho[x.x & kRay];
+                        acc = fmaf(coef(x), __fadd_rn(rv.x, rv.y), acc);
                     }
-                    const float s2 = __fadd_rn(a2, __shfl_xor_sync(kAllLanes, a2, 1));
-                    for (int q = 0; q < min(most - r, kPairs); ++q) h = __fadd_rn(h, __shfl_sync(kAllLanes, s2, 2 * q));
-                }
-                const float delta = xi ? -1.0f : 1.0f;
-                const float t = __fadd_rn(__uint_as_float(rb.x), h);
-                const float prior = __fmul_rn(A.lambda, float(int(rb.w) - 2 * unlike));
-                const float dE = __fadd_rn(__fadd_rn(__fmul_rn(delta, t), __uint_as_float(rb.y)), prior);
-                const bool flip = nsg && (dE <= 0.0f || uphill_accept(u53, double(dE), T, inv_T));
-                if (flip) {
+                    if (heavy) {
 #pragma unroll
-                    for (int u = 0; u < kHold; ++u)   // rho += delta a'
-                        rho[en[u].x & kRay] = two_sum_add(held[u], __fmul_rn(delta, __uint_as_float(en[u].y)));
-                    for (int r = kPairs; r < nsg; r += kPairs) {
-                        const int first = int(ra.x) + r * kSegE, l2 = last_of(r + pair);
-                        for (int e = half; e < l2; e += 2) {
-                            const uint2 en = __ldg(A.ent + first + e);
-                            float2& to = rho[en.x & kRay];
-                            to = two_sum_add(to, __fmul_rn(delta, __uint_as_float(en.y)));
+                        for (int off = 16; off >= 8; off >>= 1) {
+                            acc = __fadd_rn(acc, __shfl_xor_sync(kAllLanes, acc, off));
+                            unlike += __shfl_xor_sync(kAllLanes, unlike, off);
                         }
                     }
-                    if (gl == 0) {
-                        atomicXor(&xs[i >> 5], 1u << (i & 31));
-                        ++my_accepts;
-                        if (A.trace) atomicAdd(&s_trace, double(dE));
+#pragma unroll
+                    for (int off = 4; off > 0; off >>= 1) {
+                        acc = __fadd_rn(acc, __shfl_xor_sync(kAllLanes, acc, off));
+                        unlike += __shfl_xor_sync(kAllLanes, unlike, off);
+                    }
+                    const float delta = xi ? -1.0f : 1.0f;
+                    const float t = __fadd_rn(__uint_as_float(rb.x), acc);
+                    const float prior = __fmul_rn(A.lambda, float(int(rb.w) - 2 * unlike));
+                    const float dE = __fadd_rn(__fadd_rn(__fmul_rn(delta, t), __uint_as_float(rb.y)), prior);
+                    const bool flip = live && (dE <= 0.0f || uphill_accept(u53, double(dE), T, inv_T));
+                    if (flip) {
+#pragma unroll
+                        for (int u = 0; u < kHold; ++u)
+                            rho[en[u].x & kRay] = two_sum_add(held[u], __fmul_rn(delta, __uint_as_float(en[u].y)));
+                        for (int e = gl + G * kHold; e < rays; e += G) {
+                            const uint2 x = __ldg(A.ent + ra.x + e);
+                            float2& to = rho[x.x & kRay];
+                            to = two_sum_add(to, __fmul_rn(delta, __uint_as_float(x.y)));
+                        }
+                        if (gl == 0) {
+                            atomicXor(&xs[i >> 5], 1u << (i & 31));
+                            ++my_accepts;
+                            if (A.trace) atomicAdd(&s_trace, double(dE));
+                        }
+                    }
+                } else {
+                    const uint32_t tag = ra.y;
+                    const int nsg = int(tag >> 16), base = 2 * int((tag >> 5) & 31u);
+                    const int i = int(ra.z);
+                    float2 held[kHold];
+#pragma unroll
+                    for (int u = 0; u < kHold; ++u) held[u] = rho[en[u].x & kRay];
+                    const uint32_t xi = bit_of(i);
+                    int unlike = 0;
+#pragma unroll
+                    for (int t = 0; t < kNbrLane; ++t)
+                        if (nbr[t] >= 0) unlike += int(bit_of(nbr[t]) ^ xi);
+                    const int gl = lane - base;
+                    if (nsg && gl < 2)
+                        for (int j = gl + 2 * kNbrLane; j < int(rb.w); j += 2) unlike += int(bit_of(__ldg(A.nbr + rb.z + j)) ^ xi);
+                    float acc = 0.0f;
+#pragma unroll
+                    for (int u = 0; u < kHold; ++u) acc = fmaf(coef(en[u]), __fadd_rn(held[u].x, held[u].y), acc);
+                    const float seg = __fadd_rn(acc, __shfl_xor_sync(kAllLanes, acc, 1));
+                    unlike += __shfl_xor_sync(kAllLanes, unlike, 1);
+                    unlike = __shfl_sync(kAllLanes, unlike, base);
+                    // the bit's segment sums in order
+                    const int most = int(__reduce_max_sync(kAllLanes, unsigned(nsg)));
+                    float h = 0.0f;
+                    for (int q0 = 0; q0 < min(most, kPairs); q0 += 4) {
+                        float v[4];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) v[q] = __shfl_sync(kAllLanes, seg, (base + 2 * (q0 + q)) & 31);
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+                            if (q0 + q < min(nsg, kPairs)) h = __fadd_rn(h, v[q]);
+                    }
+                    // a bit of more segments has the warp to itself: further rounds
+                    auto last_of = [&](int q) { return q == nsg - 1 ? int((tag >> 10) & 31u) : q < nsg ? kSegE : 0; };
+                    for (int r = kPairs; r < most; r += kPairs) {
+                        const int first = int(ra.x) + r * kSegE, l2 = last_of(r + pair);
+                        float a2 = 0.0f;
+                        for (int e = half; e < l2; e += 2) {
+                            const uint2 en = __ldg(A.ent + first + e);
+                            const float2 rv = rho[en.x & kRay];
+                            a2 = fmaf(coef(en), __fadd_rn(rv.x, rv.y), a2);
+                        }
+                        const float s2 = __fadd_rn(a2, __shfl_xor_sync(kAllLanes, a2, 1));
+                        for (int q = 0; q < min(most - r, kPairs); ++q) h = __fadd_rn(h, __shfl_sync(kAllLanes, s2, 2 * q));
+                    }
+                    const float delta = xi ? -1.0f : 1.0f;
+                    const float t = __fadd_rn(__uint_as_float(rb.x), h);
+                    const float prior = __fmul_rn(A.lambda, float(int(rb.w) - 2 * unlike));
+                    const float dE = __fadd_rn(__fadd_rn(__fmul_rn(delta, t), __uint_as_float(rb.y)), prior);
+                    const bool flip = nsg && (dE <= 0.0f || uphill_accept(u53, double(dE), T, inv_T));
+                    if (flip) {
+#pragma unroll
+                        for (int u = 0; u < kHold; ++u)   // rho += delta a'
+                            rho[en[u].x & kRay] = two_sum_add(held[u], __fmul_rn(delta, __uint_as_float(en[u].y)));
+                        for (int r = kPairs; r < nsg; r += kPairs) {
+                            const int first = int(ra.x) + r * kSegE, l2 = last_of(r + pair);
+                            for (int e = half; e < l2; e += 2) {
+                                const uint2 en = __ldg(A.ent + first + e);
+                                float2& to = rho[en.x & kRay];
+                                to = two_sum_add(to, __fmul_rn(delta, __uint_as_float(en.y)));
+                            }
+                        }
+                        if (gl == 0) {
+                            atomicXor(&xs[i >> 5], 1u << (i & 31));
+                            ++my_accepts;
+                            if (A.trace) atomicAdd(&s_trace, double(dE));
+                        }
                     }
                 }
                 it0 += kLocalWarps;
@@ -315,7 +390,47 @@ size_t local_smem(int n, int n_rays, int n_colours) {
 
 bool resid_local_fit(int n, int n_rays, int n_colours) { return n_rays >= 1 && local_smem(n, n_rays, n_colours) <= kLocalSmem; }
 
+static void group_plan(ResidualPlan& P) {
+    P.l_rec.clear();
+    P.l_ptr.assign(1, 0);
+    int items = 0;
+    auto put = [&](int k, int at, bool heavy) {
+        uint32_t* r = &P.l_rec[(size_t(items - 1) * kGroupRecs + size_t(at)) * 8];
+        const int row = P.h_row[size_t(k)];
+        r[0] = uint32_t(row);
+        r[1] = uint32_t(P.h_row[size_t(k) + 1] - row) | kLiveTag | (heavy ? kHeavyTag : 0u);
+        r[2] = uint32_t(k);
+        r[3] = uint32_t(P.col.order[size_t(k)]);
+        std::memcpy(r + 4, &P.h_lin[size_t(k)], 4);
+        std::memcpy(r + 5, &P.h_q[size_t(k)], 4);
+        r[6] = uint32_t(P.h_nbr_ptr[size_t(k)]);
+        r[7] = uint32_t(P.h_nbr_ptr[size_t(k) + 1] - P.h_nbr_ptr[size_t(k)]);
+    };
+    auto open_item = [&]() {
+        ++items;
+        P.l_rec.resize(size_t(items) * kGroupRecs * 8, 0u);
+    };
+    for (int c = 0; c < P.col.n_colours(); ++c) {
+        int at = kGroupRecs;
+        for (int k = P.col.class_ptr[size_t(c)]; k < P.col.class_ptr[size_t(c) + 1]; ++k)
+            if (P.h_row[size_t(k) + 1] - P.h_row[size_t(k)] > kHeavyRays) {
+                open_item();
+                for (int q = 0; q < kGroupRecs; ++q) put(k, q, true);
+            }
+        for (int k = P.col.class_ptr[size_t(c)]; k < P.col.class_ptr[size_t(c) + 1]; ++k) {
+            if (P.h_row[size_t(k) + 1] - P.h_row[size_t(k)] > kHeavyRays) continue;
+            if (at == kGroupRecs) {
+                open_item();
+                at = 0;
+            }
+            put(k, at++, false);
+        }
+        P.l_ptr.push_back(items);
+    }
+}
+
 void resid_local_plan(ResidualPlan& P) {
+    if (P.variant == QB_RESID_CLUSTER) return group_plan(P);
     P.l_rec.clear();
     P.l_ptr.assign(1, 0);
     const int nc = P.col.n_colours();
@@ -378,12 +493,14 @@ void resid_local_plan(ResidualPlan& P) {
 bool resid_local_route(const ResidualPlan& p, int R) {
     if (!p.local || std::getenv("QB_PHASE_TIMES") || std::getenv("QB_TEST_BARRIER_STALL")) return false;
     const char* k = std::getenv("QB_RESID_KERNEL");
-    if (k && std::strcmp(k, "lockstep") == 0) return false;
+    if (k && (std::strcmp(k, "lockstep") == 0 || std::strcmp(k, "cluster") == 0)) return false;
     if (k && std::strcmp(k, "local") == 0) return true;
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const double classes = p.col.n_colours(), items = p.l_ptr.empty() ? 0.0 : p.l_ptr.back();
     const double local = std::max(1.05 * classes, 0.1 * items) * ((R + sms - 1) / sms);
+    // the cluster sweep: 3.3 a class step (5,000 bits, 18 branches, one CTA a branch)
+    if (p.variant == QB_RESID_CLUSTER) return std::max(1.05 * classes, 0.1 * items) < 3.3 * classes;
     double lock = 0.0;
     for (int left = R; left > 0; left -= resid_lockstep_max_branches()) {
         const int groups = (std::min(left, resid_lockstep_max_branches()) + 15) / 16;
@@ -417,8 +534,9 @@ qb_status launch_resid_local(const ResidualPlan& p, const SolveBuffers& b, int R
     A.drift = b.drift;
     A.accepts = b.accepts;
     A.trace = b.trace;
-    QB_CUDA(allow_max_smem(resid_local_kernel));
-    resid_local_kernel<<<unsigned(R), kLocalThreads, local_smem(p.n, p.n_rays, A.n_colours), st>>>(A);
+    auto kern = p.variant == QB_RESID_CLUSTER ? resid_local_kernel<true> : resid_local_kernel<false>;
+    QB_CUDA(allow_max_smem(kern));
+    kern<<<unsigned(R), kLocalThreads, local_smem(p.n, p.n_rays, A.n_colours), st>>>(A);
     QB_CUDA(cudaGetLastError());
     return QB_OK;
 }

@@ -1,5 +1,5 @@
 // The residual sweep of a problem whose branch fits one CTA's shared memory
-// (qb_local.cu), in the lockstep sweep's arithmetic.
+// (qb_local.cu), in the lockstep or the cluster sweep's arithmetic as planned.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -9,7 +9,7 @@
 
 namespace qb {
 
-// Whether a lockstep-planned problem's branch (residual pairs, bits) fits.
+// Whether a problem's branch (residual pairs, bits) fits.
 bool resid_local_fit(int n, int n_rays, int n_colours);
 // The work table of the local sweep (host): per class, warp items of 16 lane
 // pairs, a pair per 16-entry segment, a bit's pairs side by side.

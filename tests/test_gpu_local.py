@@ -1,12 +1,12 @@
-"""The residual sweep with a CTA per branch against the lockstep sweep and the
-oracle, bit for bit: empty and single rays, bits without rays, bits of one to
+"""The residual sweep with a CTA per branch against the lockstep and the cluster
+sweep and the oracle, bit for bit: empty and single rays, bits without rays, bits of one to
 more than sixteen segments, more branches than SMs, negative weights, long
 neighbour lists, the refresh, traces."""
 import numpy as np
 import pytest
 
 from oracle import oracle as O
-from qublar_b200 import ResidualProblem, Schedule, synth
+from qublar_b200 import OPT_RESID_CLUSTER, ResidualProblem, Schedule, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -44,17 +44,18 @@ CASES = {
 }
 
 
+@pytest.mark.parametrize("order", ["lockstep", "cluster"])
 @pytest.mark.parametrize("name", list(CASES))
-def test_equals_the_lockstep_sweep_and_the_oracle(name, monkeypatch):
+def test_equals_the_planned_sweep_and_the_oracle(name, order, monkeypatch):
     make, R, sweeps = CASES[name]
     arr = make()
-    P = ResidualProblem.from_arrays(arr)
+    P = ResidualProblem.from_arrays(arr, flags=OPT_RESID_CLUSTER if order == "cluster" else 0)
     s = Schedule(20.0, 0.6, sweeps, 6, 11)
     monkeypatch.setenv("QB_RESID_KERNEL", "local")
     r = P.solve(s, R, 3, trace=True)
     u = P.solve(s, R, 3)   # without the trace: class barriers across sweeps too
     assert (u.branches() == r.branches()).all()
-    monkeypatch.setenv("QB_RESID_KERNEL", "lockstep")
+    monkeypatch.setenv("QB_RESID_KERNEL", order)
     o = P.solve(s, R, 3, trace=True)
     monkeypatch.delenv("QB_RESID_KERNEL")
     X = r.branches()
@@ -64,8 +65,8 @@ def test_equals_the_lockstep_sweep_and_the_oracle(name, monkeypatch):
     assert a.accepted == b.accepted and a.max_drift == b.max_drift
     scale = np.maximum(1.0, np.abs(o.energy_trace()).max())
     assert np.abs(r.energy_trace() - o.energy_trace()).max() <= 1e-12 * sweeps * scale   # fp64 sums in another order
-    order, _ = P.colouring()
+    visits, _ = P.colouring()
     temps = O.temperatures(s.t_hot, s.t_cold, s.anneal_sweeps, s.hold_sweeps)
     for k in (0, R - 1):
-        x, _ = O.resid_anneal_coloured(arr, order, temps, s.refresh_sweeps, k + 4, mode=1)
+        x, _ = O.resid_anneal_coloured(arr, visits, temps, s.refresh_sweeps, k + 4, mode=P.info().variant)
         assert (X[k] == x).all(), k
