@@ -1230,8 +1230,9 @@ extern "C" qb_status qb_schedule_scaled(const qb_problem* p, int32_t anneal_swee
 
 // The sweep an ising solve takes (all give the same branches): few replicas
 // and dense graphs (qb_replica.cu), many replicas of one coupling size
+// (qb_word.cu), large graphs of one coupling size on the whole device
 // (qb_word.cu), otherwise a CTA per replica with its fields (qb_kernels.cu).
-enum class IsingRoute { kReplicas, kWords, kFields };
+enum class IsingRoute { kGrid, kReplicas, kWords, kFields };
 
 extern "C" qb_status qb_solve(qb_problem* p, const qb_schedule* sch, uint32_t n_branches, uint64_t seed_offset,
                               const qb_opts* opts, qb_result** out) {
@@ -1310,16 +1311,23 @@ extern "C" qb_status qb_solve(qb_problem* p, const qb_schedule* sch, uint32_t n_
             if ((s = alloc_async(r->d_f, size_t(R) * size_t(n) * 4, st))) return bail(s);
             if ((s = alloc_async(r->d_e_i64, size_t(R) * 8, st))) return bail(s);
             if ((s = alloc_async(r->d_e_scr, size_t(R) * 8, st))) return bail(s);
-            const IsingRoute route = replica_solve_fit(P, R, std::max(sch->t_hot, sch->t_cold)) ? IsingRoute::kReplicas
+            const IsingRoute route = !b.trace && word_grid_fit(P, R) && !word_solve_fit(P, R) ? IsingRoute::kGrid
+                                     : replica_solve_fit(P, R, std::max(sch->t_hot, sch->t_cold)) ? IsingRoute::kReplicas
                                      : !b.trace && word_solve_fit(P, R)                        ? IsingRoute::kWords
                                                                                                : IsingRoute::kFields;
+            if (route == IsingRoute::kGrid) {
+                if ((s = alloc_async(r->d_scratch, word_grid_scratch(P, R), st))) return bail(s);
+                r->d_err = reinterpret_cast<const int*>(static_cast<const char*>(r->d_scratch.p) + 16);
+            }
             if (route == IsingRoute::kFields && ising_smem_bytes(P) == 0 &&
                 (s = alloc_async(r->d_scratch, size_t(R) * size_t(n) * 5, st))) return bail(s);
             b.f = r->d_f.as<int32_t>();
             b.e_i64 = r->d_e_i64.as<long long>();
             b.scratch = r->d_scratch.p;
             cudaEventRecord(r->ev0, st);
-            if (route == IsingRoute::kReplicas) {
+            if (route == IsingRoute::kGrid) {
+                s = launch_word_grid(P, b.x, b.f, b.e_i64, b.temp, R, r->sweeps, seed0, r->d_scratch.p, st);
+            } else if (route == IsingRoute::kReplicas) {
                 s = launch_ising_replicas(P, b, R, r->sweeps, seed0, st);
             } else if (route == IsingRoute::kWords) {
                 AsyncAllocScope scope(st);

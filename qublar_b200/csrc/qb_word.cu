@@ -116,6 +116,18 @@ struct Butterfly {
     }
 };
 
+// Where a sweep's words live: the CTA's shared memory, or global memory that
+// other CTAs write (read past the L1 cache).
+template <typename WT>
+struct SharedWords {
+    const WT* p;
+    __device__ __forceinline__ uint32_t operator[](uint32_t j) const { return uint32_t(p[j]); }
+};
+struct GlobalWords {
+    const uint32_t* p;
+    __device__ __forceinline__ uint32_t operator[](uint32_t j) const { return __ldcg(p + j); }
+};
+
 // A lane's share of one chunk of sixteen neighbours: 16 / NP consecutive
 // entries, loaded at once. Rows are padded to sixteen with the bit itself,
 // whose word cancels; a chunk past the row is the bit itself throughout.
@@ -141,14 +153,14 @@ struct Share {
         }
     }
     // The neighbours' words against the bit's own (xr: repeated over the register), packed.
-    template <typename WT>
-    __device__ __forceinline__ uint32_t words(const WT* X, uint32_t xr) const {
+    template <typename XS>
+    __device__ __forceinline__ uint32_t words(const XS& X, uint32_t xr) const {
         constexpr int G = 2 * NP;
         uint32_t v = 0;
 #pragma unroll
         for (int t = 0; t < E; ++t) {
             const uint32_t e = sizeof(AT) == 4 || E == 1 ? w[t < W ? t : 0] : t & 1 ? w[t / 2] >> 16 : w[t / 2] & 0xFFFFu;
-            v += uint32_t(X[e]) << (t * G);
+            v += X[e] << (t * G);
         }
         return v ^ xr;
     }
@@ -213,8 +225,8 @@ __device__ __forceinline__ void count_chunks(const Butterfly<NP>& bf, const uint
     }
 }
 
-template <int NP, int K, typename AT, typename WT>
-__device__ __forceinline__ void count_ahead(const Butterfly<NP>& bf, const Ahead<NP, AT>& ah, const WT* X, uint32_t xr,
+template <int NP, int K, typename AT, typename XS>
+__device__ __forceinline__ void count_ahead(const Butterfly<NP>& bf, const Ahead<NP, AT>& ah, const XS& X, uint32_t xr,
                                             int& ca, int& cb) {
     uint32_t v[K];
 #pragma unroll
@@ -225,17 +237,17 @@ __device__ __forceinline__ void count_ahead(const Butterfly<NP>& bf, const Ahead
 // For the warp's bits (lane = (bit, pair p)): the number of neighbours j of
 // bit i with v_j = 1 in replicas 2p (ca) and 2p + 1 (cb). The first chunks'
 // entries are in `ah`.
-template <int NP, typename AT, typename WT>
-__device__ __forceinline__ void count_pair(const Butterfly<NP>& bf, const WT* X, const AT* __restrict__ row, int deg,
+template <int NP, typename AT, typename XS>
+__device__ __forceinline__ void count_pair(const Butterfly<NP>& bf, const XS& X, const AT* __restrict__ row, int deg,
                                            uint32_t self, uint32_t xi, const Ahead<NP, AT>& ah, int& ca, int& cb) {
     constexpr int K = Ahead<NP, AT>::K;
     const uint32_t xr = repeated<2 * NP>(xi);
     const int chunks = (__reduce_max_sync(kAll, deg) + 15) >> 4;
     ca = cb = 0;
-    if (K == 1 || chunks <= 1) count_ahead<NP, 1, AT, WT>(bf, ah, X, xr, ca, cb);
-    else if (K == 2 || chunks == 2) count_ahead<NP, (K > 1 ? 2 : 1), AT, WT>(bf, ah, X, xr, ca, cb);
-    else if (chunks == 3) count_ahead<NP, (K > 2 ? 3 : 1), AT, WT>(bf, ah, X, xr, ca, cb);
-    else count_ahead<NP, K, AT, WT>(bf, ah, X, xr, ca, cb);
+    if (K == 1 || chunks <= 1) count_ahead<NP, 1, AT, XS>(bf, ah, X, xr, ca, cb);
+    else if (K == 2 || chunks == 2) count_ahead<NP, (K > 1 ? 2 : 1), AT, XS>(bf, ah, X, xr, ca, cb);
+    else if (chunks == 3) count_ahead<NP, (K > 2 ? 3 : 1), AT, XS>(bf, ah, X, xr, ca, cb);
+    else count_ahead<NP, K, AT, XS>(bf, ah, X, xr, ca, cb);
     for (int u = K; u < chunks; u += 3) {   // longer rows: three chunks at a time
         Share<NP, AT> s[3];
 #pragma unroll
@@ -332,7 +344,7 @@ __device__ __forceinline__ void word_item(int team, int tid, int threads, uint32
                 const int deg = int(rec.y);
                 const uint32_t xi = uint32_t(X[i]);
                 int ca, cb;
-                count_pair<NP, AT, WT>(bf, X, row_of(rec), deg, packed_self<NP, AT>(i), xi, ah, ca, cb);
+                count_pair<NP, AT>(bf, SharedWords<WT>{X}, row_of(rec), deg, packed_self<NP, AT>(i), xi, ah, ca, cb);
                 const uint32_t oi = rec.z;
                 rec = rn;
                 ah.load(row_of(rec), int(rec.y), packed_self<NP, AT>(ni));
@@ -376,7 +388,7 @@ __device__ __forceinline__ void word_item(int team, int tid, int threads, uint32
             const int deg = int(rec.y);
             const uint32_t xi = uint32_t(X[i]);
             int ca, cb;
-            count_pair<NP, AT, WT>(bf, X, row_of(rec), deg, packed_self<NP, AT>(i), xi, ah, ca, cb);
+            count_pair<NP, AT>(bf, SharedWords<WT>{X}, row_of(rec), deg, packed_self<NP, AT>(i), xi, ah, ca, cb);
             if (valid) {
                 const size_t o = size_t(rec.z);
                 const int da = w0 * (2 * ca - deg), db = w0 * (2 * cb - deg);   // = -s_i f_i
@@ -430,6 +442,139 @@ __global__ void __launch_bounds__(kWordThreads, 1) ising_word_kernel(const WordI
             }
         }
         __syncthreads();
+    }
+}
+
+// One problem on the whole device: words of 32 replicas in global memory, a
+// cooperative grid whose warps visit a class's bits (two per pass) for every
+// group of 32 replicas, a bounded grid barrier behind each class. For few
+// replicas of a large graph, where a CTA per replica leaves most SMs idle.
+// Bound: the class step's latency, a grid barrier (1.4 us) and the pass behind
+// it (L2 gathers). 60,000 bits of degree 5, 32 replicas x 100 sweeps on a B200:
+// 15.5 ms with a CTA per replica, 2.9 here.
+struct GridArgs {
+    const int32_t* class_ptr;
+    const uint4* rec;
+    const void* adj;
+    const double* temp;
+    uint32_t* X;          // groups x 2 n words: values, complements
+    long long* e_out;     // R (zeroed)
+    uint8_t* x_out;
+    int32_t* f_out;
+    unsigned* bar;
+    int* err;
+    uint64_t seed0;
+    long long f0_sum;
+    int n;
+    int n_colours;
+    int sweeps;
+    int R;
+    int groups;
+    int w0;
+    int max_deg;
+};
+
+constexpr int kGridThreads = 1024;
+
+template <typename AT>
+__global__ void __launch_bounds__(kGridThreads, 1) ising_grid_kernel(GridArgs A) {
+    constexpr int NP = 16, BW = 2;
+    __shared__ unsigned long long s_thr[2 * kWordMaxDegree + 1];
+    __shared__ long long s_e[32];
+    const int n = A.n, nc = A.n_colours, max_deg = A.max_deg;
+    unsigned long long* thr = s_thr + max_deg;
+    const int tid = int(threadIdx.x), lane = tid & 31, q = lane & (NP - 1), sub = lane / NP;
+    const int gw = __shfl_sync(kAll, int(blockIdx.x) * (kGridThreads / 32) + (tid >> 5), 0);
+    const int tw = int(gridDim.x) * (kGridThreads / 32);
+    const AT* __restrict__ adj = static_cast<const AT*>(A.adj);
+    const Butterfly<NP> bf(q);
+    auto row_of = [&](const uint4& r) { return adj + size_t(r.x) * 16 + q; };
+    for (size_t k = size_t(blockIdx.x) * kGridThreads + tid; k < size_t(A.groups) * 2 * size_t(n);
+         k += size_t(gridDim.x) * kGridThreads)
+        __stcg(A.X + k, (k / size_t(n)) & 1 ? kAll : 0u);
+    for (int m = tid; m <= max_deg; m += kGridThreads) thr[-m] = ~0ull;
+    unsigned round = 0;
+    bool ok = grid_barrier(A.bar, A.err, ++round);
+    Ahead<NP, AT> ah;
+    for (int sweep = 0; ok && sweep < A.sweeps; ++sweep) {
+        const double T = A.temp[sweep];
+        for (int m = tid + 1; m <= max_deg; m += kGridThreads) thr[m] = draw_limit(A.w0 * m, T);
+        __syncthreads();
+        for (int c = 0; ok && c < nc; ++c) {
+            const int c0 = __ldg(A.class_ptr + c), c1 = __ldg(A.class_ptr + c + 1);
+            const int passes = (c1 - c0 + BW - 1) / BW;
+            for (int p = gw; p < passes * A.groups; p += tw) {
+                const int g = p / passes, base = c0 + (p - g * passes) * BW;
+                const bool valid = base + sub < c1;
+                const int i = valid ? base + sub : c1 - 1;
+                const uint4 rec = __ldg(A.rec + i);
+                const int deg = int(rec.y);
+                const uint32_t self = packed_self<NP, AT>(i);
+                ah.load(row_of(rec), deg, self);
+                uint32_t* X = A.X + size_t(g) * 2 * size_t(n);
+                const uint32_t xi = __ldcg(X + i);
+                const uint64_t key = A.seed0 + uint64_t(32 * g) + uint64_t(2 * q);
+                const Philox4 d = philox4x32_10(rec.z, uint32_t(sweep), 0u, 0u, uint32_t(key), uint32_t(key >> 32));
+                int ca, cb;
+                count_pair<NP, AT>(bf, GlobalWords{X}, row_of(rec), deg, self, xi, ah, ca, cb);
+                const unsigned long long za = (uint64_t(d.v[1]) << 32) | uint64_t(d.v[0] & ~2047u);
+                const unsigned long long zb = (uint64_t(d.v[3]) << 32) | uint64_t(d.v[2] & ~2047u);
+                const unsigned ba = __ballot_sync(kAll, valid && za < thr[2 * ca - deg]);
+                const unsigned bb = __ballot_sync(kAll, valid && zb < thr[2 * cb - deg]);
+                if (q == 0 && valid) {
+                    const uint32_t x = xi ^ __byte_perm(ba, bb, sub ? 0x7632 : 0x5410);
+                    __stcg(X + i, x);
+                    __stcg(X + n + i, ~x);
+                }
+            }
+            ok = grid_barrier(A.bar, A.err, ++round);
+        }
+    }
+    if (!ok) return;
+    // fields and energies from the final words, as in word_item
+    const int passes = (n + BW - 1) / BW;
+    for (int g = 0; g < A.groups; ++g) {
+        if (tid < 32) s_e[tid] = 0;
+        __syncthreads();
+        const int ra = 32 * g + 2 * q, rb = ra + 1;
+        long long Ea = 0, Eb = 0;
+        for (int p = gw; p < passes; p += tw) {
+            const bool valid = p * BW + sub < n;
+            const int i = valid ? p * BW + sub : n - 1;
+            const uint4 rec = __ldg(A.rec + i);
+            const int deg = int(rec.y);
+            const uint32_t self = packed_self<NP, AT>(i);
+            ah.load(row_of(rec), deg, self);
+            const uint32_t* X = A.X + size_t(g) * 2 * size_t(n);
+            const uint32_t xi = __ldcg(X + i);
+            int ca, cb;
+            count_pair<NP, AT>(bf, GlobalWords{X}, row_of(rec), deg, self, xi, ah, ca, cb);
+            if (!valid) continue;
+            const size_t o = size_t(rec.z);
+            const int da = A.w0 * (2 * ca - deg), db = A.w0 * (2 * cb - deg);
+            const int xa = int((xi >> q) & 1u), xb = int((xi >> (q + NP)) & 1u);
+            Ea -= da;
+            Eb -= db;
+            if (ra < A.R) {
+                A.x_out[size_t(ra) * size_t(n) + o] = uint8_t(xa);
+                A.f_out[size_t(ra) * size_t(n) + o] = xa ? -da : da;
+            }
+            if (rb < A.R) {
+                A.x_out[size_t(rb) * size_t(n) + o] = uint8_t(xb);
+                A.f_out[size_t(rb) * size_t(n) + o] = xb ? -db : db;
+            }
+        }
+        if (Ea) atomicAdd(reinterpret_cast<unsigned long long*>(&s_e[2 * q]), (unsigned long long)Ea);
+        if (Eb) atomicAdd(reinterpret_cast<unsigned long long*>(&s_e[2 * q + 1]), (unsigned long long)Eb);
+        __syncthreads();
+        if (tid < 32 && 32 * g + tid < A.R && s_e[tid])
+            atomicAdd(reinterpret_cast<unsigned long long*>(&A.e_out[32 * g + tid]), (unsigned long long)s_e[tid]);
+        __syncthreads();
+    }
+    if (!grid_barrier(A.bar, A.err, ++round)) return;
+    for (int r = int(blockIdx.x) * kGridThreads + tid; r < A.R; r += int(gridDim.x) * kGridThreads) {
+        const long long e = (long long)atomicAdd(reinterpret_cast<unsigned long long*>(&A.e_out[r]), 0ull);
+        A.e_out[r] = (e + A.f0_sum) / 4;
     }
 }
 
@@ -655,6 +800,46 @@ qb_status launch_word_solve(const IsingPlan& p, uint8_t* x, int32_t* f, long lon
     QB_CUDA(cudaMemcpyAsync(base + kCtl + ib, w.bundles.data(), bb, cudaMemcpyHostToDevice, st));
     return launch_ising_words(w, reinterpret_cast<const WordItem*>(base + kCtl),
                               reinterpret_cast<const WordBundle*>(base + kCtl + ib), reinterpret_cast<int*>(base), st);
+}
+
+// Large graphs of few classes: a class step of the whole device costs about 2.7
+// us, a sweep of the CTA-per-replica kernels about 2.3 ns a bit (26,000 bits, 5
+// classes: 60 us against 14).
+bool word_grid_fit(const IsingPlan& p, int R) {
+    return word_sweep(p) && int64_t(p.n) * ((R + 31) / 32) < (int64_t(1) << 30) && p.n >= 2000 * p.col.n_colours() && !std::getenv("QB_ISING_THREADS");
+}
+
+size_t word_grid_scratch(const IsingPlan& p, int R) { return 256 + size_t((R + 31) / 32) * 2 * size_t(p.n) * 4; }
+
+qb_status launch_word_grid(const IsingPlan& p, uint8_t* x, int32_t* f, long long* e, const double* temp, int R, int sweeps,
+                           uint64_t seed0, void* scratch, cudaStream_t st) {
+    GridArgs A{};
+    A.class_ptr = p.d_class_ptr.as<int32_t>();
+    A.rec = p.d_wrec.as<uint4>();
+    A.adj = p.d_wadj.p;
+    A.temp = temp;
+    A.bar = static_cast<unsigned*>(scratch);
+    A.err = reinterpret_cast<int*>(static_cast<char*>(scratch) + 16);
+    A.X = reinterpret_cast<uint32_t*>(static_cast<char*>(scratch) + 256);
+    A.e_out = e;
+    A.x_out = x;
+    A.f_out = f;
+    A.seed0 = seed0;
+    A.f0_sum = p.f0_sum;
+    A.n = p.n;
+    A.n_colours = p.col.n_colours();
+    A.sweeps = sweeps;
+    A.R = R;
+    A.groups = (R + 31) / 32;
+    A.w0 = int32_t(p.max_w);
+    A.max_deg = p.max_deg;
+    QB_CUDA(cudaMemsetAsync(scratch, 0, 256, st));
+    QB_CUDA(cudaMemsetAsync(e, 0, size_t(R) * 8, st));
+    const void* kern = p.word_bytes() == 4 ? reinterpret_cast<const void*>(ising_grid_kernel<uint32_t>)
+                                           : reinterpret_cast<const void*>(ising_grid_kernel<uint16_t>);
+    void* args[] = {&A};
+    QB_CUDA(cudaLaunchCooperativeKernel(kern, dim3(unsigned(word_sms())), dim3(kGridThreads), args, 0, st));
+    return QB_OK;
 }
 
 }  // namespace qb

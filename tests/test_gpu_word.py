@@ -99,3 +99,18 @@ def test_many_replicas_equal_the_cta_per_replica_sweep(R, monkeypatch):
     o = P.solve(b, R, 4)
     assert (r.branches() == o.branches()).all() and (r.fields() == o.fields()).all()
     assert (r.energies_tracked() == o.energies_tracked()).all() and (r.energies() == o.energies()).all()
+
+
+@pytest.mark.parametrize("n,d,R", [(32700, 3, 33), (40001, 3, 70), (33000, 5, 1), (90000, 4, 32)])
+def test_whole_device_words_equal_the_field_sweep(n, d, R, monkeypatch):
+    """Large graphs of few classes: words in global memory on a cooperative grid."""
+    g = synth.random_regular(n, d, 3) if n != 90000 else synth.torus_pm1(300, 5)
+    P = IsingProblem(*g)
+    assert P.n >= 2000 * P.info().n_colours
+    s = P.scaled_schedule(9, 1)
+    r = P.solve(s, R, 12)
+    monkeypatch.setenv("QB_ISING_THREADS", "512")
+    o = P.solve(s, R, 12)
+    assert (r.branches() == o.branches()).all() and (r.fields() == o.fields()).all()
+    assert (r.energies_tracked() == o.energies_tracked()).all() and (r.energies() == o.energies()).all()
+    assert (r.marginals() == o.marginals()).all()
