@@ -1559,6 +1559,7 @@ extern "C" qb_status qb_energies_ising(const qb_problem* p, const uint8_t* x, in
         if (!p->uploaded) return fail(QB_EINVAL, "qb_energies_ising: the problem is not on the device");
         if (k == 0) return QB_OK;
         QB_CUDA(cudaSetDevice(p->device));
+        AsyncAllocScope scope(nullptr);   // the buffers from the library's pool
         DevBuf dx, de;
         qb_status s;
         if ((s = upload(dx, x, size_t(k) * size_t(p->ising.n), nullptr))) return s;
@@ -1576,6 +1577,7 @@ extern "C" qb_status qb_energies_qubo(const qb_problem* p, const uint8_t* x, int
         if (!p->uploaded) return fail(QB_EINVAL, "qb_energies_qubo: the problem is not on the device");
         if (k == 0) return QB_OK;
         QB_CUDA(cudaSetDevice(p->device));
+        AsyncAllocScope scope(nullptr);   // the buffers from the library's pool
         DevBuf dx, de;
         qb_status s;
         if ((s = upload(dx, x, size_t(k) * size_t(p->qubo.n), nullptr))) return s;
@@ -1593,6 +1595,7 @@ extern "C" qb_status qb_energies_residual(const qb_problem* p, const uint8_t* x,
         if (!p->uploaded) return fail(QB_EINVAL, "qb_energies_residual: the problem is not on the device");
         if (k == 0) return QB_OK;
         QB_CUDA(cudaSetDevice(p->device));
+        AsyncAllocScope scope(nullptr);   // the buffers from the library's pool
         DevBuf dx, de;
         qb_status s;
         if ((s = upload(dx, x, size_t(k) * size_t(p->resid.n), nullptr))) return s;
