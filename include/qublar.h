@@ -346,7 +346,11 @@ typedef struct qb_batch_item {
 } qb_batch_item;
 
 /* Launch shape of the packed kernel; zeros take the defaults (512 threads,
- * 96 KiB of state per CTA, groups of up to 32 replicas). */
+ * 96 KiB of state per CTA, groups of up to 32 replicas). Instances of one
+ * coupling size (every |w| equal) with four or more branches run as words of
+ * replicas in a launch of their own, to which threads, max_group and ctas do
+ * not apply; a non-zero smem_bytes that does not hold their n x 5 bytes keeps
+ * them on the launch shaped here. */
 typedef struct qb_batch_config {
     int32_t threads;         /* per CTA: a multiple of 32 in [32, 1024] */
     int32_t smem_bytes;      /* shared memory for one item's state (n x group x 5 bytes) */

@@ -1311,7 +1311,7 @@ extern "C" qb_status qb_solve(qb_problem* p, const qb_schedule* sch, uint32_t n_
             if ((s = alloc_async(r->d_f, size_t(R) * size_t(n) * 4, st))) return bail(s);
             if ((s = alloc_async(r->d_e_i64, size_t(R) * 8, st))) return bail(s);
             if ((s = alloc_async(r->d_e_scr, size_t(R) * 8, st))) return bail(s);
-            const IsingRoute route = !b.trace && word_grid_fit(P, R) && !word_solve_fit(P, R) ? IsingRoute::kGrid
+            const IsingRoute route = !b.trace && word_grid_fit(P, R, r->sweeps) && !word_solve_fit(P, R) ? IsingRoute::kGrid
                                      : replica_solve_fit(P, R, std::max(sch->t_hot, sch->t_cold)) ? IsingRoute::kReplicas
                                      : !b.trace && word_solve_fit(P, R)                        ? IsingRoute::kWords
                                                                                                : IsingRoute::kFields;

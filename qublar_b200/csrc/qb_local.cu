@@ -206,7 +206,8 @@ __global__ void __launch_bounds__(kLocalThreads, 1) resid_local_kernel(ResidLoca
     };
     bool ready = s0 == 0 && c0 == 0;   // nothing to wait for before the item in hand
     unsigned long long my_accepts = 0;
-    for (int sweep = 0; sweep < A.sweeps; ++sweep) {
+    int turn = 0;   // sweep x classes modulo 15
+    for (int sweep = 0; sweep < A.sweeps; ++sweep, turn = (turn + nc) % 15) {
         if (full_stop(sweep)) {
             __syncthreads();
             if (A.trace && tid == 0) {   // the sweep before
@@ -235,8 +236,8 @@ __global__ void __launch_bounds__(kLocalThreads, 1) resid_local_kernel(ResidLoca
         const double T = A.temp[sweep];
         const float inv_T = float(1.0 / T);
         while (s0 == sweep && total > 0) {
-            const int c = c0, idx = sweep * nc + c;
-            if (!ready && !(c == 0 && full_stop(sweep))) wait_class(idx - 1, members(c > 0 ? c - 1 : nc - 1));
+            const int c = c0, idx = turn + c;   // the barrier behind class c, modulo 15
+            if (!ready && !(c == 0 && full_stop(sweep))) wait_class(idx + 15 - 1, members(c > 0 ? c - 1 : nc - 1));
             do {   // the warp's items of this class
                 if constexpr (GROUPS) {
                     const bool heavy = (ra.y & kHeavyTag) != 0, live = (ra.y & kLiveTag) != 0;   // heavy: warp-uniform
@@ -394,6 +395,7 @@ static void group_plan(ResidualPlan& P) {
     P.l_rec.clear();
     P.l_ptr.assign(1, 0);
     int items = 0;
+    P.l_rec.reserve(size_t(P.n) * 9);
     auto put = [&](int k, int at, bool heavy) {
         uint32_t* r = &P.l_rec[(size_t(items - 1) * kGroupRecs + size_t(at)) * 8];
         const int row = P.h_row[size_t(k)];
@@ -436,6 +438,7 @@ void resid_local_plan(ResidualPlan& P) {
     const int nc = P.col.n_colours();
     auto segs = [&](int k) { return std::max(1, (P.h_row[size_t(k) + 1] - P.h_row[size_t(k)] + kSegE - 1) / kSegE); };
     int items = 0;
+    P.l_rec.reserve((size_t(P.nnz) / kSegE + size_t(P.n)) * 8);
     auto open_item = [&]() {
         ++items;
         P.l_rec.resize(size_t(items) * kPairs * 8, 0u);

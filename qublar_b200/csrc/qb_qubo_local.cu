@@ -137,7 +137,8 @@ __global__ void __launch_bounds__(32 * kSmallMaxWarps, 1) qubo_small_kernel(Qubo
     bool ready = s0 == 0 && c0 == 0;
     float eh = 0.0f, el = 0.0f, drift = 0.0f;
     unsigned long long accepts = 0;
-    for (int sweep = 0; sweep < A.sweeps; ++sweep) {
+    int turn = 0;   // sweep x classes modulo kBarriers
+    for (int sweep = 0; sweep < A.sweeps; ++sweep, turn = (turn + nc) % kBarriers) {
         if (full_stop(sweep)) {
             __syncthreads();
             if (tid < R) {
@@ -150,8 +151,8 @@ __global__ void __launch_bounds__(32 * kSmallMaxWarps, 1) qubo_small_kernel(Qubo
         const float inv_T = float(1.0 / T);
         const bool refresh = A.refresh > 0 && sweep > 0 && sweep % A.refresh == 0;
         while (s0 == sweep) {
-            const int c = c0, idx = sweep * nc + c;
-            if (!ready && !(c == 0 && full_stop(sweep))) wait_class(idx - 1, members(c > 0 ? c - 1 : nc - 1));
+            const int c = c0, idx = turn + c;   // the barrier behind class c, modulo kBarriers
+            if (!ready && !(c == 0 && full_stop(sweep))) wait_class(idx + kBarriers - 1, members(c > 0 ? c - 1 : nc - 1));
             do {
                 if (!A.ahead) load_state();
                 float hi = own.x, lo = own.y;

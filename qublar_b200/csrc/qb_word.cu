@@ -805,8 +805,10 @@ qb_status launch_word_solve(const IsingPlan& p, uint8_t* x, int32_t* f, long lon
 // Large graphs of few classes: a class step of the whole device costs about 2.7
 // us, a sweep of the CTA-per-replica kernels about 2.3 ns a bit (26,000 bits, 5
 // classes: 60 us against 14).
-bool word_grid_fit(const IsingPlan& p, int R) {
-    return word_sweep(p) && int64_t(p.n) * ((R + 31) / 32) < (int64_t(1) << 30) && p.n >= 2000 * p.col.n_colours() && !std::getenv("QB_ISING_THREADS");
+// The barrier's counter holds 2^32 arrivals, the pass index 2^31.
+bool word_grid_fit(const IsingPlan& p, int R, int sweeps) {
+    return word_sweep(p) && int64_t(p.n) * ((R + 31) / 32) < (int64_t(1) << 30) &&
+           int64_t(sweeps) * p.col.n_colours() < (int64_t(1) << 24) && p.n >= 2000 * p.col.n_colours() && !std::getenv("QB_ISING_THREADS");
 }
 
 size_t word_grid_scratch(const IsingPlan& p, int R) { return 256 + size_t((R + 31) / 32) * 2 * size_t(p.n) * 4; }

@@ -103,7 +103,7 @@ qb_status launch_ising_words(const WordWork& work, const WordItem* items, const 
 // done; x, f, e: R x n, R x n, R).
 // A single solve of a large graph on the whole device (scratch: word_grid_scratch
 // bytes, the barrier's timeout flag at +16).
-bool word_grid_fit(const IsingPlan& p, int R);
+bool word_grid_fit(const IsingPlan& p, int R, int sweeps);
 size_t word_grid_scratch(const IsingPlan& p, int R);
 qb_status launch_word_grid(const IsingPlan& p, uint8_t* x, int32_t* f, long long* e, const double* temp, int R, int sweeps,
                            uint64_t seed0, void* scratch, cudaStream_t st);
