@@ -197,6 +197,19 @@ void qb_problem_destroy(qb_problem* p);
  * waits for `device` and hands the memory the pool holds back to the driver. */
 qb_status qb_device_trim(int32_t device);
 
+/* How often this process has launched a sweep kernel, by name, or -1 for an
+ * unknown name (diagnostics: which kernel a call took follows from its sizes):
+ *   ising_fields              a CTA per replica, its fields on chip or in memory;
+ *   ising_replica_w8, _w32    few replicas, 1- and 4-byte couplings (_far: the
+ *                             adjacency in global memory); ising_dense;
+ *   ising_word_16, _32        replicas as words, 2- and 4-byte adjacency;
+ *   ising_grid_16, _32        the same on the whole device;
+ *   ising_batch, _replay      the packed kernel, launched or replayed by a graph;
+ *   resid_lockstep_1 .. _4    by branch groups; resid_cluster; resid_local and
+ *                             resid_local_cluster (in the cluster sweep's order);
+ *   qubo_lockstep, qubo_small. */
+int64_t qb_sweep_launches(const char* kernel);
+
 typedef struct qb_problem_info {
     int32_t kind;           /* QB_KIND_* */
     int32_t n;              /* bits */

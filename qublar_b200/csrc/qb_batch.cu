@@ -403,6 +403,7 @@ qb_status launch_ising_batch(const IsingItem* d_items, int n_items, int* d_count
     batch_kernel(sh.threads)<<<dim3(unsigned(ctas)), dim3(unsigned(sh.threads)), size_t(sh.smem_bytes), st>>>(d_items, n_items,
                                                                                                       d_counter);
     QB_CUDA(cudaGetLastError());
+    count_sweep(Sweep::kIsingBatch);
     return QB_OK;
 }
 

@@ -1,6 +1,8 @@
 // Status codes and the thread-local error message of the C ABI. The reference
 // exits on a CUDA error (src/ising_gpu.cuh:44-52); the library reports it.
+#include <atomic>
 #include <cstdio>
+#include <cstring>
 #include <mutex>
 #include <string>
 
@@ -50,6 +52,17 @@ cudaMemPool_t library_pool(int dev) {
     }
     return pools[dev];
 }
+
+namespace {
+const char* const kSweepNames[int(Sweep::kCount)] = {
+    "ising_fields", "ising_replica_w8", "ising_replica_w32", "ising_replica_w8_far", "ising_replica_w32_far",
+    "ising_dense", "ising_word_16", "ising_word_32", "ising_grid_16", "ising_grid_32", "ising_batch",
+    "ising_batch_replay", "resid_lockstep_1", "resid_lockstep_2", "resid_lockstep_3", "resid_lockstep_4",
+    "resid_cluster", "resid_local", "resid_local_cluster", "qubo_lockstep", "qubo_small"};
+std::atomic<int64_t> g_sweeps[int(Sweep::kCount)];
+}  // namespace
+
+void count_sweep(Sweep s) { g_sweeps[int(s)].fetch_add(1, std::memory_order_relaxed); }
 
 void set_error(const std::string& msg) { g_last_error = msg; }
 
@@ -113,6 +126,12 @@ extern "C" const char* qb_status_string(qb_status s) {
 }
 
 extern "C" const char* qb_last_error(void) { return qb::g_last_error.c_str(); }
+
+extern "C" int64_t qb_sweep_launches(const char* kernel) {
+    for (int k = 0; kernel && k < int(qb::Sweep::kCount); ++k)
+        if (std::strcmp(kernel, qb::kSweepNames[k]) == 0) return qb::g_sweeps[k].load(std::memory_order_relaxed);
+    return -1;
+}
 
 extern "C" int32_t qb_abi_version(void) { return QUBLAR_ABI_VERSION; }
 

@@ -46,6 +46,17 @@ qb_status cuda_fail(cudaError_t e, const char* what, const char* file, int line)
         if (e_ != cudaSuccess) return ::qb::cuda_fail(e_, #call, __FILE__, __LINE__); \
     } while (0)
 
+// ---- launch counts --------------------------------------------------------------
+
+// The sweep kernels, in the order of kSweepNames (qb_errors.cpp).
+enum class Sweep : int {
+    kIsingFields, kIsingReplica8, kIsingReplica32, kIsingReplica8Far, kIsingReplica32Far, kIsingDense, kIsingWord16,
+    kIsingWord32, kIsingGrid16, kIsingGrid32, kIsingBatch, kIsingBatchReplay, kResidLockstep1, kResidLockstep2,
+    kResidLockstep3, kResidLockstep4, kResidCluster, kResidLocal, kResidLocalCluster, kQuboLockstep, kQuboSmall, kCount
+};
+// One more launch of a sweep kernel (qb_sweep_launches).
+void count_sweep(Sweep s);
+
 // ---- device buffer (RAII, library-owned) -------------------------------------
 
 // Allocations of a DevBuf are stream-ordered (from the library's pool on

@@ -1128,6 +1128,7 @@ qb_status launch_ising_anneal(const IsingPlan& p, const SolveBuffers& b, int R, 
         else ising_anneal_kernel<int32_t, false><<<grid, block, 0, st>>>(A);
     }
     QB_CUDA(cudaGetLastError());
+    count_sweep(Sweep::kIsingFields);
     return QB_OK;
 }
 
@@ -1239,6 +1240,7 @@ qb_status launch_resid_anneal(const ResidualPlan& p, const SolveBuffers& b, int 
         case 16: s = resid_launch_cl<16>(A, R, smem, st, false); break;
         default: return fail(QB_EINVAL, "residual sweep: cluster size must be 1, 2, 4, 8 or 16");
     }
+    if (s == QB_OK) count_sweep(Sweep::kResidCluster);
     if (s == QB_OK && phases) {
         std::vector<unsigned long long> h(size_t(R) * size_t(p.CL) * 4);
         QB_CUDA(cudaMemcpyAsync(h.data(), phase.p, phase.bytes, cudaMemcpyDeviceToHost, st));
@@ -1399,6 +1401,7 @@ qb_status launch_resid_lockstep(const ResidualPlan& p, const SolveBuffers& b, in
     const void* kern = phases ? lockstep_kernel<true>(A.NG) : lockstep_kernel<false>(A.NG);
     void* args[] = {&A};
     QB_CUDA(cudaLaunchCooperativeKernel(kern, dim3(unsigned(grid)), dim3(kLockThreads), args, resid_lockstep_smem(A.NG), st));
+    count_sweep(Sweep(int(Sweep::kResidLockstep1) + A.NG - 1));
     if (phases) {
         std::vector<unsigned long long> h(size_t(grid) * 8);
         QB_CUDA(cudaMemcpyAsync(h.data(), phase.p, phase.bytes, cudaMemcpyDeviceToHost, st));

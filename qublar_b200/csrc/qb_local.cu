@@ -541,6 +541,7 @@ qb_status launch_resid_local(const ResidualPlan& p, const SolveBuffers& b, int R
     QB_CUDA(allow_max_smem(kern));
     kern<<<unsigned(R), kLocalThreads, local_smem(p.n, p.n_rays, A.n_colours), st>>>(A);
     QB_CUDA(cudaGetLastError());
+    count_sweep(p.variant == QB_RESID_CLUSTER ? Sweep::kResidLocalCluster : Sweep::kResidLocal);
     return QB_OK;
 }
 

@@ -285,6 +285,7 @@ qb_status launch_qubo_lockstep(const QuboPlan& p, const QuboBuffers& b, int R, i
     void* args[] = {&A};
     QB_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(qubo_lockstep_kernel), dim3(unsigned(grid)),
                                         dim3(kQThreads), args, 0, st));
+    count_sweep(Sweep::kQuboLockstep);
     return QB_OK;
 }
 

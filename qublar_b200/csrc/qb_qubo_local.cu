@@ -289,6 +289,7 @@ qb_status launch_qubo_small(const QuboPlan& p, const QuboBuffers& b, int R, int 
     QB_CUDA(allow_max_smem(qubo_small_kernel));
     qubo_small_kernel<<<unsigned((R + 31) / 32), 32 * A.warps, small_smem(p), st>>>(A);
     QB_CUDA(cudaGetLastError());
+    count_sweep(Sweep::kQuboSmall);
     return QB_OK;
 }
 

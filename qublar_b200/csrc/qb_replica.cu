@@ -34,6 +34,7 @@
 #include <cstdlib>
 
 #include "qb_device.cuh"
+#include "qb_internal.hpp"
 #include "qb_kernels.hpp"
 #include "qb_philox.cuh"
 #include "qb_word.hpp"
@@ -476,6 +477,7 @@ qb_status launch_ising_replicas(const IsingPlan& p, const SolveBuffers& b, int R
         QB_CUDA(allow_max_smem(kd));
         kd<<<unsigned(R), 128, bytes, st>>>(A);
         QB_CUDA(cudaGetLastError());
+        count_sweep(Sweep::kIsingDense);
         return QB_OK;
     }
     // consumer warps: a few bits of an average class each, so that the flips'
@@ -522,6 +524,8 @@ qb_status launch_ising_replicas(const IsingPlan& p, const SolveBuffers& b, int R
     cfg.attrs = attr;
     cfg.numAttrs = A.cluster > 1 ? 1 : 0;
     QB_CUDA(cudaLaunchKernelEx(&cfg, kern, A));
+    count_sweep(p.weight_bytes == 1 ? (csr ? Sweep::kIsingReplica8 : Sweep::kIsingReplica8Far)
+                                    : (csr ? Sweep::kIsingReplica32 : Sweep::kIsingReplica32Far));
     return QB_OK;
 }
 

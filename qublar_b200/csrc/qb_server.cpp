@@ -574,11 +574,13 @@ qb_status launch_items(qb_server* S, const std::vector<IsingItem>& items) {
         QB_CUDA(cudaGraphExecMemcpyNodeSetParams1D(S->exec, S->copy_node, S->d_tick.p, S->h_tick, bytes,
                                                    cudaMemcpyHostToDevice));
         QB_CUDA(cudaGraphLaunch(S->exec, S->tick_stream));
+        count_sweep(Sweep::kIsingBatchReplay);
     } else {
         QB_CUDA(cudaMemcpyAsync(S->d_tick.p, S->h_tick, bytes, cudaMemcpyHostToDevice, S->tick_stream));
         if ((s = launch_ising_batch_ctl(reinterpret_cast<const IsingItem*>(S->d_tick.as<unsigned char>() + kTickHeader),
                                         S->d_tick.as<int>(), S->shape, S->tick_stream)))
             return s;
+        count_sweep(Sweep::kIsingBatch);
     }
     return QB_OK;
 }

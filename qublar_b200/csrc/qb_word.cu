@@ -738,6 +738,7 @@ qb_status launch_width(const WordItem* items, const WordBundle* bundles, int n, 
     QB_CUDA(allow_max_smem(ising_word_kernel<AT>));
     ising_word_kernel<AT><<<std::min(word_sms(), n), kWordThreads, sizeof(WordHead) + smem, st>>>(items, bundles, n, counter);
     QB_CUDA(cudaGetLastError());
+    count_sweep(sizeof(AT) == 2 ? Sweep::kIsingWord16 : Sweep::kIsingWord32);
     return QB_OK;
 }
 }  // namespace
@@ -841,6 +842,7 @@ qb_status launch_word_grid(const IsingPlan& p, uint8_t* x, int32_t* f, long long
                                            : reinterpret_cast<const void*>(ising_grid_kernel<uint16_t>);
     void* args[] = {&A};
     QB_CUDA(cudaLaunchCooperativeKernel(kern, dim3(unsigned(word_sms())), dim3(kGridThreads), args, 0, st));
+    count_sweep(p.word_bytes() == 4 ? Sweep::kIsingGrid32 : Sweep::kIsingGrid16);
     return QB_OK;
 }
 

@@ -57,6 +57,22 @@ def test_status_strings_and_version():
     assert L.qb_status_string(0) == b"ok"
 
 
+def test_sweep_launch_counts_by_name():
+    """The documented names are known, others refused."""
+    text = open(os.path.join(INCLUDE, "qublar.h")).read()
+    doc = re.search(r"/\* How often this process has launched(.*?)\*/", text, flags=re.S).group(1)
+    for name in ("ising_fields", "ising_dense", "resid_cluster", "resid_local", "qubo_lockstep", "qubo_small"):
+        assert name in doc
+    for name in ("ising_fields", "ising_replica_w8", "ising_replica_w32", "ising_replica_w8_far", "ising_replica_w32_far",
+                 "ising_dense", "ising_word_16", "ising_word_32", "ising_grid_16", "ising_grid_32", "ising_batch",
+                 "ising_batch_replay", "resid_lockstep_1", "resid_lockstep_2", "resid_lockstep_3", "resid_lockstep_4",
+                 "resid_cluster", "resid_local", "resid_local_cluster", "qubo_lockstep", "qubo_small"):
+        assert qb.sweep_launches(name) >= 0
+    for name in ("", "ising", "qb_nothing"):
+        with pytest.raises(ValueError):
+            qb.sweep_launches(name)
+
+
 def _ising_status(n, eu, ev, ew):
     eu, ev, ew = (np.ascontiguousarray(x, np.int32) for x in (eu, ev, ew))
     d = IsingDesc(n, eu.size, ptr(eu), ptr(ev), ptr(ew))
