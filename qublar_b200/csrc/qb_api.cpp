@@ -56,8 +56,8 @@ qb_status alloc_async(DevBuf& b, size_t bytes, cudaStream_t st) {
     return QB_OK;
 }
 
-// Stream-ordered release of a stream-ordered allocation; a buffer taken from
-// a plain allocation (the packed-replica arenas) is freed plainly.
+// Stream-ordered release of a stream-ordered allocation; one made plainly is
+// freed plainly.
 void free_async(DevBuf& b, cudaStream_t st) {
     if (b.p) {
         if (b.pooled) cudaFreeAsync(b.p, st);

@@ -195,11 +195,12 @@ struct Work {
 };
 
 // Splits every instance into replica groups for the shape `c`, sorts the
-// units largest first and writes their descriptors. sample > 0 replaces each
+// units largest first and writes their descriptors. words: whether instances may
+// run as word units. sample > 0 replaces each
 // schedule by `sample` of its sweeps, evenly spaced (autotuning), read from
 // sample_temp (one table of `sample` entries per instance).
-qb_status build_items(qb_batch* b, const qb_batch_config& c, bool smem_asked, int sample, const double* sample_temp,
-                      Work& work) {
+qb_status build_items(qb_batch* b, const qb_batch_config& c, bool words, bool smem_asked, int sample,
+                      const double* sample_temp, Work& work) {
     std::vector<IsingItem>& out = work.items;
     // instances of one coupling size run as words (qb_word.cu). A shared-memory
     // bound that the caller gave is a bound on an instance's int32 state: one
@@ -207,7 +208,7 @@ qb_status build_items(qb_batch* b, const qb_batch_config& c, bool smem_asked, in
     const size_t word_cap = word_max_smem();
     auto as_words = [&](const qb_batch::Inst& I) {
         const IsingPlan& P = I.prob->ising;
-        return word_sweep(P) && I.R >= kWordMinReplicas && word_item_smem(P, 2) <= word_cap &&
+        return words && word_sweep(P) && I.R >= kWordMinReplicas && word_item_smem(P, 2) <= word_cap &&
                !(smem_asked && batch_item_smem(I.n, 1) > size_t(c.smem_bytes));
     };
     double total = 0.0;
@@ -353,6 +354,50 @@ qb_status item_of(qb_batch* b, int32_t item, const void* dst) {
     return wait(b);
 }
 
+// words: whether instances of one coupling size may run as word units (else
+// every instance runs on the launch that cfg shapes).
+qb_status solve_batch(const qb_batch_item* items, int32_t count, const qb_batch_config* cfg, const qb_opts* opts, bool words,
+                      qb_batch** out) {
+    if (!out) return fail(QB_EINVAL, "qb_solve_batch: null output");
+    *out = nullptr;
+    qb_status s = check_items(items, count);
+    if (s != QB_OK) return s;
+    qb_batch_config c{};
+    if ((s = resolve_config(cfg, &c)) != QB_OK) return s;
+    QB_CUDA(cudaSetDevice(items[0].problem->device));
+    const int cap = batch_max_smem();
+    if (cap <= 0) return fail(QB_ECUDA, "batch: cannot read the device's shared-memory limit");
+    c.smem_bytes = std::min(c.smem_bytes, cap);
+    qb_batch* b = new (std::nothrow) qb_batch();
+    if (!b) return fail(QB_ENOMEM, "qb_solve_batch: out of host memory");
+    auto bail = [&](qb_status e) {
+        qb_batch_destroy(b);
+        return e;
+    };
+    // the batch's memory from the library's pool; qb_batch_destroy waits for the stream first
+    AsyncAllocScope scope(opts ? static_cast<cudaStream_t>(opts->stream) : nullptr, true);
+    if ((s = prepare(items, count, opts, b)) != QB_OK) return bail(s);
+    b->cfg = c;
+    Work work;
+    if ((s = build_items(b, c, words, cfg && cfg->smem_bytes != 0, 0, nullptr, work)) != QB_OK) return bail(s);
+    b->work_items = int(work.items.size() + work.words.items.size());
+    if (cudaEventCreate(&b->ev0) != cudaSuccess || cudaEventCreate(&b->ev1) != cudaSuccess ||
+        cudaEventCreate(&b->ev2) != cudaSuccess)
+        return bail(cuda_fail(cudaGetLastError(), "cudaEventCreate", __FILE__, __LINE__));
+    // the descriptors go up before the timed region
+    if ((s = upload_work(b, work)) != QB_OK) return bail(s);
+    cudaEventRecord(b->ev0, b->stream);
+    if ((s = launch_work(b, c, work)) != QB_OK) return bail(s);
+    cudaEventRecord(b->ev1, b->stream);
+    if ((s = launch_batch_marginals(b->d_x.as<uint8_t>(), b->d_inst.as<BatchInstDev>(), int(b->inst.size()),
+                                    b->total_bits, b->d_p.as<float>(), b->stream)))
+        return bail(s);
+    cudaEventRecord(b->ev2, b->stream);
+    ++b->launches;
+    *out = b;
+    return QB_OK;
+}
+
 std::mutex g_tune_mu;
 std::map<std::tuple<int, int64_t, int64_t, int64_t, int>, qb_batch_config> g_tuned;
 
@@ -427,7 +472,7 @@ extern "C" qb_status qb_batch_autotune(const qb_batch_item* items, int32_t count
                 for (int g : group_c) {
                     qb_batch_config c{th, std::min(sm, cap), g, 0};
                     Work its;
-                    if ((s = build_items(b, c, true, S, d_st.as<double>(), its)) != QB_OK) break;
+                    if ((s = build_items(b, c, true, true, S, d_st.as<double>(), its)) != QB_OK) break;
                     float ms = 0.0f;
                     if ((s = time_shape(c, its, &ms)) != QB_OK) break;
                     if (ms >= 0.0f) timed.emplace_back(ms, c);
@@ -450,7 +495,7 @@ extern "C" qb_status qb_batch_autotune(const qb_batch_item* items, int32_t count
             s = upload_vec(d_st4, st4, b->stream);
             for (size_t q = 0; s == QB_OK && q < std::min<size_t>(3, timed.size()); ++q) {
                 Work its;
-                if ((s = build_items(b, timed[q].second, true, S4, d_st4.as<double>(), its)) != QB_OK) break;
+                if ((s = build_items(b, timed[q].second, true, true, S4, d_st4.as<double>(), its)) != QB_OK) break;
                 float ms = 0.0f;
                 if ((s = time_shape(timed[q].second, its, &ms)) != QB_OK) break;
                 if (ms >= 0.0f && (best < 0.0f || ms < best)) {
@@ -475,46 +520,7 @@ extern "C" qb_status qb_batch_autotune(const qb_batch_item* items, int32_t count
 
 extern "C" qb_status qb_solve_batch(const qb_batch_item* items, int32_t count, const qb_batch_config* cfg,
                                     const qb_opts* opts, qb_batch** out) {
-    return qb::guarded("qb_solve_batch", [&]() -> qb_status {
-        if (!out) return fail(QB_EINVAL, "qb_solve_batch: null output");
-        *out = nullptr;
-        qb_status s = check_items(items, count);
-        if (s != QB_OK) return s;
-        qb_batch_config c{};
-        if ((s = resolve_config(cfg, &c)) != QB_OK) return s;
-        QB_CUDA(cudaSetDevice(items[0].problem->device));
-        const int cap = batch_max_smem();
-        if (cap <= 0) return fail(QB_ECUDA, "batch: cannot read the device's shared-memory limit");
-        c.smem_bytes = std::min(c.smem_bytes, cap);
-        qb_batch* b = new (std::nothrow) qb_batch();
-        if (!b) return fail(QB_ENOMEM, "qb_solve_batch: out of host memory");
-        auto bail = [&](qb_status e) {
-            qb_batch_destroy(b);
-            return e;
-        };
-        // the batch's memory from the library's pool; qb_batch_destroy waits for the stream first
-        AsyncAllocScope scope(opts ? static_cast<cudaStream_t>(opts->stream) : nullptr, true);
-        if ((s = prepare(items, count, opts, b)) != QB_OK) return bail(s);
-        b->cfg = c;
-        Work work;
-        if ((s = build_items(b, c, cfg && cfg->smem_bytes != 0, 0, nullptr, work)) != QB_OK) return bail(s);
-        b->work_items = int(work.items.size() + work.words.items.size());
-        if (cudaEventCreate(&b->ev0) != cudaSuccess || cudaEventCreate(&b->ev1) != cudaSuccess ||
-            cudaEventCreate(&b->ev2) != cudaSuccess)
-            return bail(cuda_fail(cudaGetLastError(), "cudaEventCreate", __FILE__, __LINE__));
-        // the descriptors go up before the timed region
-        if ((s = upload_work(b, work)) != QB_OK) return bail(s);
-        cudaEventRecord(b->ev0, b->stream);
-        if ((s = launch_work(b, c, work)) != QB_OK) return bail(s);
-        cudaEventRecord(b->ev1, b->stream);
-        if ((s = launch_batch_marginals(b->d_x.as<uint8_t>(), b->d_inst.as<BatchInstDev>(), int(b->inst.size()),
-                                        b->total_bits, b->d_p.as<float>(), b->stream)))
-            return bail(s);
-        cudaEventRecord(b->ev2, b->stream);
-        ++b->launches;
-        *out = b;
-        return QB_OK;
-    });
+    return qb::guarded("qb_solve_batch", [&]() -> qb_status { return solve_batch(items, count, cfg, opts, true, out); });
 }
 
 extern "C" qb_status qb_batch_info_get(qb_batch* b, qb_batch_info* info) {
@@ -621,7 +627,7 @@ qb_status packed_replicas(qb_problem* p, const qb_schedule& s, int R, uint64_t s
     const qb_batch_item item{p, s, uint32_t(R), seed_offset};
     qb_batch_config cfg{kPackedThreads, sh.smem_bytes, G, 0};
     qb_batch* b = nullptr;
-    if ((st = qb_solve_batch(&item, 1, &cfg, opts, &b)) != QB_OK) return st;
+    if ((st = solve_batch(&item, 1, &cfg, opts, false, &b)) != QB_OK) return st;
     take(x, b->d_x);
     take(f, b->d_f);
     take(e, b->d_e);

@@ -10,7 +10,7 @@ import numpy as np
 import pytest
 
 from oracle import oracle as O
-from qublar_b200 import Budget, IsingProblem, autotune_batch, solve_batch, synth
+from qublar_b200 import Budget, IsingProblem, autotune_batch, solve_batch, sweep_launches, synth
 from qublar_b200._abi import BatchConfig
 
 pytestmark = pytest.mark.gpu
@@ -126,12 +126,13 @@ def test_many_replicas_route_equals_the_cta_per_replica_sweep(monkeypatch):
     """qb_solve with 128 or more replicas (QB_PACKED_REPLICAS=1) runs them as
     work items of the packed kernel; branches, tracked energies, fields and
     marginals equal those of one CTA per replica, whatever the CTA size."""
-    from qublar_b200 import Budget
     n, eu, ev, ew = synth.erdos_renyi(800, 0.06, 1)
     P = IsingProblem(n, eu, ev, ew)
     b = Budget(3.0, 0.05, 100, 0)
     monkeypatch.setenv("QB_PACKED_REPLICAS", "1")
+    packed = sweep_launches("ising_batch")
     r = P.solve(b, 256, 7)
+    assert sweep_launches("ising_batch") == packed + 1   # one coupling size too, not the word sweep
     X, E, F, p = r.branches(), r.energies_tracked(), r.fields(), r.marginals()
     monkeypatch.delenv("QB_PACKED_REPLICAS")
     for threads in ("512", "128"):
