@@ -362,8 +362,8 @@ typedef struct qb_batch_item {
  * 96 KiB of state per CTA, groups of up to 32 replicas). Instances of one
  * coupling size (every |w| equal) with four or more branches run as words of
  * replicas in a launch of their own, to which threads, max_group and ctas do
- * not apply; a non-zero smem_bytes that does not hold their n x 5 bytes keeps
- * them on the launch shaped here. */
+ * not apply; a smem_bytes of 1 to 48 KiB that does not hold their n x 5 bytes
+ * keeps them on the launch shaped here, with their state in device memory. */
 typedef struct qb_batch_config {
     int32_t threads;         /* per CTA: a multiple of 32 in [32, 1024] */
     int32_t smem_bytes;      /* shared memory for one item's state (n x group x 5 bytes) */
@@ -371,12 +371,13 @@ typedef struct qb_batch_config {
     int32_t ctas;            /* persistent CTAs; 0 = as many as fit the device */
 } qb_batch_config;
 
-/* Times candidate shapes on the batch itself with its schedules sampled at
- * sample_sweeps evenly spaced sweeps (0 = 8), times the three fastest again
- * on a sample four times longer, and returns the fastest of those. The
- * answer is kept per process for batches of the same shape (instance count,
- * total bits, total edges, total branches) and returned at once next time.
- * Results do not depend on the shape. */
+/* Times candidate shapes on the batch's instances that the packed kernel runs,
+ * with their schedules sampled at sample_sweeps evenly spaced sweeps (0 = 8),
+ * times the three fastest again on a sample four times longer, and returns the
+ * fastest of those; a batch without such instances takes the defaults. The
+ * answer is kept per process for batches whose such instances have the same
+ * count, total bits, total edges and total branches, and returned at once next
+ * time. Results do not depend on the shape. */
 qb_status qb_batch_autotune(const qb_batch_item* items, int32_t count, int32_t sample_sweeps, const qb_opts* opts,
                             qb_batch_config* out);
 

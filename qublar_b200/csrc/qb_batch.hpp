@@ -59,6 +59,18 @@ struct BatchShape {
 // Shared memory one item of n bits and G replicas needs.
 inline size_t batch_item_smem(int n, int G) { return size_t(n) * size_t(G) * 5; }
 
+// Word units narrower than four replicas leave most of a pass's Philox lanes
+// to replicas that do not exist; the field-carrying kernel serves those.
+constexpr int kWordMinReplicas = 4;
+// The largest qb_batch_config.smem_bytes that is a caller's request for global
+// state: an instance of one coupling size whose int32 state of one replica it
+// does not hold stays off the word sweep. The tuner's shapes lie above it, so a
+// tuned configuration takes no instance off its faster sweep.
+constexpr int kStateBound = 48 * 1024;
+// Whether R replicas of an instance run as word units (qb_word.cu). bound: the
+// smem_bytes that the caller gave (0: none); word_cap: word_max_smem().
+bool batch_as_words(const IsingPlan& p, int R, int bound, size_t word_cap);
+
 // Largest dynamic shared memory a CTA of the packed kernel can take.
 int batch_max_smem();
 // Persistent CTAs that fit the device at this shape.

@@ -54,9 +54,6 @@ namespace {
 constexpr int kDefaultThreads = 512;
 constexpr int kDefaultSmem = 96 * 1024;
 constexpr int kDefaultGroup = 32;
-// Word units narrower than four replicas leave most of a pass's Philox lanes
-// to replicas that do not exist; the field-carrying kernel serves those.
-constexpr int kWordMinReplicas = 4;
 // The largest word unit, as a share of one SM's part of the whole batch: large
 // instances are split over their replicas until no unit outlasts the others
 // (128 mixed instances of 200 to 20,000 bits, 200 sweeps: 21.6 ms at 1.0, 25.7
@@ -196,20 +193,16 @@ struct Work {
 
 // Splits every instance into replica groups for the shape `c`, sorts the
 // units largest first and writes their descriptors. words: whether instances may
-// run as word units. sample > 0 replaces each
+// run as word units; bound: the smem_bytes that the caller gave (0: none).
+// sample > 0 replaces each
 // schedule by `sample` of its sweeps, evenly spaced (autotuning), read from
 // sample_temp (one table of `sample` entries per instance).
-qb_status build_items(qb_batch* b, const qb_batch_config& c, bool words, bool smem_asked, int sample,
+qb_status build_items(qb_batch* b, const qb_batch_config& c, bool words, int bound, int sample,
                       const double* sample_temp, Work& work) {
     std::vector<IsingItem>& out = work.items;
-    // instances of one coupling size run as words (qb_word.cu). A shared-memory
-    // bound that the caller gave is a bound on an instance's int32 state: one
-    // that exceeds it at a single replica runs on global state as asked.
     const size_t word_cap = word_max_smem();
     auto as_words = [&](const qb_batch::Inst& I) {
-        const IsingPlan& P = I.prob->ising;
-        return words && word_sweep(P) && I.R >= kWordMinReplicas && word_item_smem(P, 2) <= word_cap &&
-               !(smem_asked && batch_item_smem(I.n, 1) > size_t(c.smem_bytes));
+        return words && batch_as_words(I.prob->ising, I.R, bound, word_cap);
     };
     double total = 0.0;
     for (const qb_batch::Inst& I : b->inst)
@@ -379,7 +372,7 @@ qb_status solve_batch(const qb_batch_item* items, int32_t count, const qb_batch_
     if ((s = prepare(items, count, opts, b)) != QB_OK) return bail(s);
     b->cfg = c;
     Work work;
-    if ((s = build_items(b, c, words, cfg && cfg->smem_bytes != 0, 0, nullptr, work)) != QB_OK) return bail(s);
+    if ((s = build_items(b, c, words, cfg ? cfg->smem_bytes : 0, 0, nullptr, work)) != QB_OK) return bail(s);
     b->work_items = int(work.items.size() + work.words.items.size());
     if (cudaEventCreate(&b->ev0) != cudaSuccess || cudaEventCreate(&b->ev1) != cudaSuccess ||
         cudaEventCreate(&b->ev2) != cudaSuccess)
@@ -412,15 +405,22 @@ extern "C" qb_status qb_batch_autotune(const qb_batch_item* items, int32_t count
         if (s0 != QB_OK) return s0;
         QB_CUDA(cudaSetDevice(items[0].problem->device));
         const int S = sample_sweeps ? sample_sweeps : 8;
+        // the shape concerns the field-carrying launch alone: its instances are
+        // timed, and a batch without any takes the defaults
+        std::vector<qb_batch_item> fields;
+        const size_t word_cap = word_max_smem();
+        for (int32_t k = 0; k < count; ++k)
+            if (!batch_as_words(items[k].problem->ising, int(items[k].n_branches), 0, word_cap)) fields.push_back(items[k]);
+        if (fields.empty()) return resolve_config(nullptr, out);
         qb_batch* b = new (std::nothrow) qb_batch();
         if (!b) return fail(QB_ENOMEM, "qb_batch_autotune: out of host memory");
         AsyncAllocScope scope(opts ? static_cast<cudaStream_t>(opts->stream) : nullptr, true);
-        qb_status s = prepare(items, count, opts, b);
+        qb_status s = prepare(fields.data(), int32_t(fields.size()), opts, b);
         if (s != QB_OK) {
             qb_batch_destroy(b);
             return s;
         }
-        const auto key = std::make_tuple(count, b->total_bits, b->total_nnz, b->total_r, b->device);
+        const auto key = std::make_tuple(int(fields.size()), b->total_bits, b->total_nnz, b->total_r, b->device);
         {
             std::lock_guard<std::mutex> lk(g_tune_mu);
             auto hit = g_tuned.find(key);
@@ -443,7 +443,7 @@ extern "C" qb_status qb_batch_autotune(const qb_batch_item* items, int32_t count
         }
         const int cap = batch_max_smem();
         const int threads_c[] = {256, 512, 1024};
-        const int smem_c[] = {48 * 1024, 96 * 1024, cap};
+        const int smem_c[] = {50 * 1024, 96 * 1024, cap};   // all above kStateBound
         const int group_c[] = {8, 16, 32};
         cudaEvent_t e0, e1;
         cudaEventCreate(&e0);
@@ -472,7 +472,7 @@ extern "C" qb_status qb_batch_autotune(const qb_batch_item* items, int32_t count
                 for (int g : group_c) {
                     qb_batch_config c{th, std::min(sm, cap), g, 0};
                     Work its;
-                    if ((s = build_items(b, c, true, true, S, d_st.as<double>(), its)) != QB_OK) break;
+                    if ((s = build_items(b, c, false, 0, S, d_st.as<double>(), its)) != QB_OK) break;
                     float ms = 0.0f;
                     if ((s = time_shape(c, its, &ms)) != QB_OK) break;
                     if (ms >= 0.0f) timed.emplace_back(ms, c);
@@ -495,7 +495,7 @@ extern "C" qb_status qb_batch_autotune(const qb_batch_item* items, int32_t count
             s = upload_vec(d_st4, st4, b->stream);
             for (size_t q = 0; s == QB_OK && q < std::min<size_t>(3, timed.size()); ++q) {
                 Work its;
-                if ((s = build_items(b, timed[q].second, true, true, S4, d_st4.as<double>(), its)) != QB_OK) break;
+                if ((s = build_items(b, timed[q].second, false, 0, S4, d_st4.as<double>(), its)) != QB_OK) break;
                 float ms = 0.0f;
                 if ((s = time_shape(timed[q].second, its, &ms)) != QB_OK) break;
                 if (ms >= 0.0f && (best < 0.0f || ms < best)) {
@@ -588,6 +588,11 @@ extern "C" void qb_batch_destroy(qb_batch* b) {
 }
 
 namespace qb {
+
+bool batch_as_words(const IsingPlan& p, int R, int bound, size_t word_cap) {
+    return word_sweep(p) && R >= kWordMinReplicas && word_item_smem(p, 2) <= word_cap &&
+           !(bound > 0 && bound <= kStateBound && batch_item_smem(p.n, 1) > size_t(bound));
+}
 
 namespace {
 constexpr int kPackedMinReplicas = 128;

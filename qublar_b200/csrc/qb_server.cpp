@@ -119,7 +119,7 @@ struct qb_server {
     int next_resid_stream = 0;
     cudaEvent_t upload_ev = nullptr, tick_ev = nullptr;
     BatchShape shape;
-    bool smem_asked = false;   // the caller bounded an ising item's shared-memory state
+    int state_bound = 0;       // the smem_bytes that the caller gave (0: none)
     DevBuf d_words;            // the tick's word units: counters, items, bundles
     unsigned char* h_words = nullptr;
     size_t words_cap = 0;
@@ -237,13 +237,9 @@ void plan_groups(qb_server* S, Request* r, double target_attempts) {
     r->slice = int(std::max(1.0, std::min(double(r->sweeps), std::floor(target_attempts / per_sweep))));
 }
 
-// Whether an ising request runs as word units (qb_word.cu): one coupling size,
-// at least four replicas, words that fit a CTA; not where the caller's bound on
-// an item's state asks for global state.
+// Whether an ising request runs as word units (qb_word.cu).
 bool as_words(const qb_server* S, const Request* r) {
-    const IsingPlan& P = r->prob->ising;
-    return word_sweep(P) && r->R >= 4 && word_item_smem(P, 2) <= word_max_smem() &&
-           !(S->smem_asked && batch_item_smem(r->n, 1) > size_t(S->shape.smem_bytes));
+    return batch_as_words(r->prob->ising, r->R, S->state_bound, word_max_smem());
 }
 
 // Bytes of a word unit's kept state.
@@ -878,7 +874,7 @@ extern "C" qb_status qb_server_create(const qb_server_config* cfg, qb_server** o
         const int cap = batch_max_smem();
         if (cap <= 0) return fail(QB_ECUDA, "qb_server_create: cannot read the shared-memory limit");
         c.batch.smem_bytes = std::min(c.batch.smem_bytes, cap);
-        S->smem_asked = cfg && cfg->batch.smem_bytes != 0;
+        S->state_bound = cfg ? cfg->batch.smem_bytes : 0;
         S->cfg = c;
         S->shape.threads = c.batch.threads;
         S->shape.smem_bytes = c.batch.smem_bytes;

@@ -145,3 +145,27 @@ def test_many_replicas_route_equals_the_cta_per_replica_sweep(monkeypatch):
     assert (q.energies_tracked() == E).all() and (q.fields() == F).all()
     assert (q.marginals() == p).all()
     assert (r.energies() == E.astype(np.float64)).all()
+
+
+def test_autotune_times_what_its_shape_concerns():
+    """A batch of word instances takes the defaults untimed; a weighted batch of
+    the same totals is timed all the same; a tuned shape takes no instance off
+    the word sweep, however large; results are those of the default shape."""
+    n, eu, ev, ew = synth.random_regular(600, 8, 3)
+    one, weighted = IsingProblem(n, eu, ev, ew), IsingProblem(n, eu, ev, np.arange(1, ew.size + 1, dtype=np.int32))
+    large = IsingProblem(*synth.random_regular(50001, 4, 2))
+    sched = one.scaled_schedule(30, 2)
+    packed = sweep_launches("ising_batch")
+    cfg = autotune_batch([(one, sched, 9, 0)])
+    assert (cfg.threads, cfg.smem_bytes, cfg.max_group) == (512, 96 * 1024, 32)
+    assert sweep_launches("ising_batch") == packed
+    autotune_batch([(weighted, sched, 9, 0)])
+    assert sweep_launches("ising_batch") > packed
+    items = [(large, large.scaled_schedule(6, 0), 5, 3), (weighted, sched, 9, 0)]
+    cfg = autotune_batch(items)
+    before = sweep_launches("ising_word_32"), sweep_launches("ising_batch")
+    B = solve_batch(items, cfg)
+    assert (sweep_launches("ising_word_32"), sweep_launches("ising_batch")) == (before[0] + 1, before[1] + 1)
+    D = solve_batch(items)
+    for k in range(2):
+        assert (B.branches(k) == D.branches(k)).all() and (B.energies_tracked(k) == D.energies_tracked(k)).all()
