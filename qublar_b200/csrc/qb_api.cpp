@@ -20,6 +20,7 @@
 #include "qb_kernels.hpp"
 #include "qb_local.hpp"
 #include "qb_qubo.hpp"
+#include "qb_route.hpp"
 #include "qb_word.hpp"
 
 using namespace qb;
@@ -1228,12 +1229,6 @@ extern "C" qb_status qb_schedule_scaled(const qb_problem* p, int32_t anneal_swee
 
 // ---- solve ---------------------------------------------------------------------------------------
 
-// The sweep an ising solve takes (all give the same branches): few replicas
-// and dense graphs (qb_replica.cu), many replicas of one coupling size
-// (qb_word.cu), large graphs of one coupling size on the whole device
-// (qb_word.cu), otherwise a CTA per replica with its fields (qb_kernels.cu).
-enum class IsingRoute { kGrid, kReplicas, kWords, kFields };
-
 extern "C" qb_status qb_solve(qb_problem* p, const qb_schedule* sch, uint32_t n_branches, uint64_t seed_offset,
                               const qb_opts* opts, qb_result** out) {
     return qb::guarded("qb_solve", [&]() -> qb_status {
@@ -1311,10 +1306,7 @@ extern "C" qb_status qb_solve(qb_problem* p, const qb_schedule* sch, uint32_t n_
             if ((s = alloc_async(r->d_f, size_t(R) * size_t(n) * 4, st))) return bail(s);
             if ((s = alloc_async(r->d_e_i64, size_t(R) * 8, st))) return bail(s);
             if ((s = alloc_async(r->d_e_scr, size_t(R) * 8, st))) return bail(s);
-            const IsingRoute route = !b.trace && word_grid_fit(P, R, r->sweeps) && !word_solve_fit(P, R) ? IsingRoute::kGrid
-                                     : replica_solve_fit(P, R, std::max(sch->t_hot, sch->t_cold)) ? IsingRoute::kReplicas
-                                     : !b.trace && word_solve_fit(P, R)                        ? IsingRoute::kWords
-                                                                                               : IsingRoute::kFields;
+            const IsingRoute route = ising_route(P, R, r->sweeps, std::max(sch->t_hot, sch->t_cold), b.trace != nullptr);
             if (route == IsingRoute::kGrid) {
                 if ((s = alloc_async(r->d_scratch, word_grid_scratch(P, R), st))) return bail(s);
                 r->d_err = reinterpret_cast<const int*>(static_cast<const char*>(r->d_scratch.p) + 16);

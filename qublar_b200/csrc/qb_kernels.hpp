@@ -31,8 +31,10 @@ struct SolveBuffers {
 size_t ising_smem_bytes(const IsingPlan& p);
 qb_status launch_ising_anneal(const IsingPlan& p, const SolveBuffers& b, int R, int sweeps, uint64_t seed0,
                               cudaStream_t st);
-// At most one replica per SM: the sweep with the draws off its chain
-// (qb_replica.cu); t_max: the schedule's largest temperature.
+// At most one replica per SM, or a dense graph of any number: the sweeps with
+// the draws off their chain (qb_replica.cu); t_max: the schedule's largest
+// temperature. dense_solve_us: the estimated time of a dense graph's solve.
+double dense_solve_us(const IsingPlan& p, int R, int sweeps);
 bool replica_solve_fit(const IsingPlan& p, int R, double t_max);
 qb_status launch_ising_replicas(const IsingPlan& p, const SolveBuffers& b, int R, int sweeps, uint64_t seed0,
                                 cudaStream_t st);

@@ -417,6 +417,9 @@ __global__ void __launch_bounds__(128) ising_dense_kernel(ReplicaArgs A) {
 // A visit costs about an eighth of a class step: dense graphs, where most
 // classes hold a few bits.
 bool dense_fit(const IsingPlan& p) { return p.n <= kDenseMax && p.n <= 8 * p.col.n_colours(); }
+size_t dense_smem(const IsingPlan& p) {
+    return (size_t(p.n) * size_t(p.n) + 2 * size_t(kDenseAhead) * size_t(p.n)) * 4;
+}
 
 int replica_ahead(const IsingPlan& p) { return std::max(1, std::min(8, 4096 / p.n)); }
 size_t replica_base_smem(const IsingPlan& p) {
@@ -432,6 +435,17 @@ constexpr double kReplicaMaxT = 0x1.0p40;
 constexpr double kStepCycles = 260.0, kDrawCycles = 1500.0;
 
 }  // namespace
+
+double dense_solve_us(const IsingPlan& p, int R, int sweeps) {
+    // a visit takes 50, 65 or 95 ns by its registers; CTAs of an SM share it
+    // from about nine on. 200 bits, 20 sweeps: 0.39 ms for 148 replicas, 1.91
+    // for 600, 10.8 for 4,096 (CTA-per-replica sweep: 2.2, 2.3 and 7.2)
+    const double visit = p.n <= 64 ? 0.050 : p.n <= 128 ? 0.065 : 0.095;
+    const int fit = std::max(1, std::min(16, int(size_t(227) * 1024 / (dense_smem(p) + 1024))));
+    const int waves = (R + word_sms() * fit - 1) / (word_sms() * fit);
+    const double resident = std::min(double(fit), std::ceil(double(R) / word_sms()));
+    return 8.0 + sweeps * (waves * p.n * visit * std::max(1.0, resident / 9.0));
+}
 
 // One wave of replicas (one CTA per SM) with the state in shared memory, or a
 // dense graph. With the CSR in global memory only classes of at most a few
@@ -469,7 +483,7 @@ qb_status launch_ising_replicas(const IsingPlan& p, const SolveBuffers& b, int R
     A.trace = reinterpret_cast<long long*>(b.trace);
     A.wbytes = p.weight_bytes;
     if (dense_fit(p)) {
-        const size_t bytes = (size_t(p.n) * size_t(p.n) + 2 * size_t(kDenseAhead) * size_t(p.n)) * 4;
+        const size_t bytes = dense_smem(p);
         void (*kd)(ReplicaArgs) = p.n <= 32    ? ising_dense_kernel<1>
                                   : p.n <= 64  ? ising_dense_kernel<2>
                                   : p.n <= 128 ? ising_dense_kernel<4>

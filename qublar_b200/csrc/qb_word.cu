@@ -32,6 +32,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 #include <cstdlib>
 #include <vector>
@@ -637,13 +638,19 @@ int word_sms() {
     return sms;
 }
 
+// Read once per device: the routes' estimates ask for it several times a call.
 size_t word_max_smem() {
+    constexpr int kDevices = 64;
+    static std::atomic<size_t> known[kDevices];
     int dev = 0, optin = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    if (dev < kDevices && known[dev].load(std::memory_order_relaxed)) return known[dev].load(std::memory_order_relaxed);
     if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return 0;
     cudaFuncAttributes fa{};
     if (cudaFuncGetAttributes(&fa, ising_word_kernel<uint16_t>) != cudaSuccess) return 0;
-    return size_t(optin) - fa.sharedSizeBytes - sizeof(WordHead);
+    const size_t most = size_t(optin) - fa.sharedSizeBytes - sizeof(WordHead);
+    if (dev < kDevices) known[dev].store(most, std::memory_order_relaxed);
+    return most;
 }
 
 // Warp instructions of one sweep: a fixed part per pass of 64 proposals
@@ -685,6 +692,27 @@ void word_fill(WordItem& it, const IsingPlan& p, int np, int live, uint64_t seed
     it.wide = p.word_bytes() == 4 ? 1 : 0;
 }
 
+namespace {
+// Teams of a CTA for a unit: split while every SM already has a unit for each
+// team and either half the team would idle through an average class or the unit
+// on its share of the SM stays below a quarter of the balanced makespan
+// (128 mixed instances: 21.6 ms at a quarter, 26.9 at the whole; 1,024
+// instances of 200 to 5,000 bits: 22.5 ms, 24.4 at a half, 28.3 at the whole)
+int word_teams(size_t smem, int passes, double cost, size_t units, double total, int sms, size_t cap) {
+    int t = 1;
+    while (t < kMaxTeams) {
+        const int t2 = 2 * t;
+        if (((smem + 15) & ~size_t(15)) * size_t(t2) > cap) break;
+        if (units <= size_t(t) * size_t(sms)) break;
+        const bool spare = 2 * passes <= kWordThreads / 32 / t;
+        const bool small = cost * t2 * sms <= 0.25 * total;
+        if (!spare && !small) break;
+        t = t2;
+    }
+    return t;
+}
+}  // namespace
+
 WordWork word_pack(std::vector<WordUnit>& units) {
     std::stable_sort(units.begin(), units.end(), [](const WordUnit& a, const WordUnit& b) {
         return a.item.wide != b.item.wide ? a.item.wide < b.item.wide : a.cost > b.cost;
@@ -694,24 +722,7 @@ WordWork word_pack(std::vector<WordUnit>& units) {
     double total = 0.0;
     for (const WordUnit& u : units) total += u.cost;
     WordWork w;
-    // teams of a unit: split while every SM already has a unit for each team
-    // and either half the team would idle through an average class or the unit
-    // on its share of the SM stays below a quarter of the balanced makespan
-    // (128 mixed instances: 21.6 ms at a quarter, 26.9 at the whole; 1,024
-    // instances of 200 to 5,000 bits: 22.5 ms, 24.4 at a half, 28.3 at the whole)
-    auto teams_of = [&](const WordUnit& u) {
-        int t = 1;
-        while (t < kMaxTeams) {
-            const int t2 = 2 * t;
-            if (((u.smem + 15) & ~size_t(15)) * size_t(t2) > cap) break;
-            if (units.size() <= size_t(t) * size_t(sms)) break;
-            const bool spare = 2 * u.passes <= kWordThreads / 32 / t;
-            const bool small = u.cost * t2 * sms <= 0.25 * total;
-            if (!spare && !small) break;
-            t = t2;
-        }
-        return t;
-    };
+    auto teams_of = [&](const WordUnit& u) { return word_teams(u.smem, u.passes, u.cost, units.size(), total, sms, cap); };
     for (size_t k = 0; k < units.size();) {
         const int t = teams_of(units[k]), wide = units[k].item.wide;
         WordBundle b{int32_t(w.items.size()), 0, t, 0};
@@ -753,28 +764,61 @@ qb_status launch_ising_words(const WordWork& work, const WordItem* items, const 
     return s;
 }
 
-// More replicas than SMs: below that the CTA-per-replica sweep has an SM for
-// each replica and its shorter class step wins. QB_ISING_THREADS asks for that
-// sweep's CTA size, hence for that sweep.
+// More replicas than SMs: below that the few-replica sweeps have an SM for each
+// replica and their shorter class step wins. QB_ISING_THREADS asks for the
+// CTA-per-replica sweep's CTA size, hence for that sweep.
 bool word_solve_fit(const IsingPlan& p, int R) {
     return word_sweep(p) && R > word_sms() && !std::getenv("QB_ISING_THREADS") &&
            word_item_smem(p, 2) <= word_max_smem();
 }
 
-qb_status launch_word_solve(const IsingPlan& p, uint8_t* x, int32_t* f, long long* e, const double* temp, int R,
-                            int sweeps, uint64_t seed0, DevBuf& tables, cudaStream_t st) {
-    // the width with the shortest estimated makespan: units per SM times their cost
+namespace {
+// The estimated microseconds of a sweep of R replicas in units of 2 np, on a
+// whole device: waves of bundles, each the longer of its chain of class steps
+// and its teams' instructions (2.2 a cycle), and a part of the other. A class
+// step is 0.42 us and 0.07 per 16 neighbours of a bit, 0.2 where the adjacency
+// exceeds the L1 cache; less in wide units on most SMs, whose lanes hold four
+// stretches at once (ER(800, 0.5), 102 classes: 4.9 us a step for 149 replicas,
+// 3.2 for 4,096; 300 bits of degree 24: 0.84).
+double word_width_us(const IsingPlan& p, int R, int np) {
+    const double nc = p.col.n_colours(), deg = double(p.nnz) / p.n;
+    const int units = (R + 2 * np - 1) / (2 * np), sms = word_sms();
+    const double cost = word_unit_cost(p.n, p.nnz, np, 1);
+    const int t = word_teams(word_item_smem(p, np), word_class_passes(p.n, p.col.n_colours(), np), cost, size_t(units),
+                             cost * units, sms, word_max_smem());
+    const int bundles = (units + t - 1) / t, waves = (bundles + sms - 1) / sms;
+    const bool far = p.nnz * p.word_bytes() > 160 * 1024, wide = np >= 8 && 2 * units >= sms;
+    const double per = far ? (wide ? 0.115 : 0.2) : (wide ? 0.045 : 0.07);
+    const double chain = nc * (0.42 + per * std::ceil(deg / 16.0));
+    const double work = std::min(t, units) * cost / 4180.0;
+    return waves * (std::max(chain, work) + 0.3 * std::min(chain, work));
+}
+
+// The width with the shortest estimate; near ties: the wider unit.
+int word_best_pairs(const IsingPlan& p, int R, double* us) {
     int np = 2;
-    double best = 0.0;
-    for (int c = 2; c <= 16; c *= 2) {
-        if (word_item_smem(p, c) > word_max_smem()) break;
-        const int units = (R + 2 * c - 1) / (2 * c);
-        const double est = double((units + word_sms() - 1) / word_sms()) * word_unit_cost(p.n, p.nnz, c, sweeps);
-        if (best == 0.0 || est < 1.02 * best) {   // near ties: the wider unit
-            best = est;
+    *us = word_width_us(p, R, 2);
+    for (int c = 4; c <= 16 && word_item_smem(p, c) <= word_max_smem(); c *= 2) {
+        const double est = word_width_us(p, R, c);
+        if (est < 1.02 * *us) {
+            *us = est;
             np = c;
         }
     }
+    return np;
+}
+}  // namespace
+
+double word_solve_us(const IsingPlan& p, int R, int sweeps) {
+    double us;
+    word_best_pairs(p, R, &us);
+    return 42.0 + sweeps * us;   // words in, fields and branches out
+}
+
+qb_status launch_word_solve(const IsingPlan& p, uint8_t* x, int32_t* f, long long* e, const double* temp, int R,
+                            int sweeps, uint64_t seed0, DevBuf& tables, cudaStream_t st) {
+    double us;
+    const int np = word_best_pairs(p, R, &us);
     std::vector<WordUnit> units;
     for (int r0 = 0; r0 < R; r0 += 2 * np) {
         WordUnit u;

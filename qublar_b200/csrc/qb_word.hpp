@@ -98,16 +98,18 @@ void word_fill(WordItem& it, const IsingPlan& p, int np, int live, uint64_t seed
 qb_status launch_ising_words(const WordWork& work, const WordItem* items, const WordBundle* bundles, int* counter,
                              cudaStream_t st);
 
-// A single solve of R replicas as word units: whether the route serves it, and
-// the launch (tables: one device allocation, kept until the stream's work is
-// done; x, f, e: R x n, R x n, R).
 // A single solve of a large graph on the whole device (scratch: word_grid_scratch
 // bytes, the barrier's timeout flag at +16).
 bool word_grid_fit(const IsingPlan& p, int R, int sweeps);
 size_t word_grid_scratch(const IsingPlan& p, int R);
 qb_status launch_word_grid(const IsingPlan& p, uint8_t* x, int32_t* f, long long* e, const double* temp, int R, int sweeps,
                            uint64_t seed0, void* scratch, cudaStream_t st);
+// A single solve of R replicas as word units: whether the route serves it, the
+// estimated time of the solve in microseconds, and the launch (tables: one
+// device allocation, kept until the stream's work is done; x, f, e: R x n, R x
+// n, R).
 bool word_solve_fit(const IsingPlan& p, int R);
+double word_solve_us(const IsingPlan& p, int R, int sweeps);
 qb_status launch_word_solve(const IsingPlan& p, uint8_t* x, int32_t* f, long long* e, const double* temp, int R,
                             int sweeps, uint64_t seed0, DevBuf& tables, cudaStream_t st);
 

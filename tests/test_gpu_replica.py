@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 from oracle import oracle as O
-from qublar_b200 import IsingProblem, Schedule, synth
+from qublar_b200 import IsingProblem, Schedule, sweep_launches, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -71,3 +71,22 @@ def test_temperatures_of_every_size(t, monkeypatch):
     monkeypatch.setenv("QB_ISING_THREADS", "64")
     o = P.solve(s, 6)
     assert (r.branches() == o.branches()).all() and (r.energies_tracked() == o.energies_tracked()).all()
+
+
+@pytest.mark.parametrize("R,kernel", [(148, "ising_dense"), (200, "ising_fields"), (1500, "ising_fields")])
+def test_dense_graphs_leave_the_dense_kernel_where_its_waves_are_longer(R, kernel):
+    """200 bits in 34 classes: one CTA of the dense kernel fills an SM, so beyond
+    one replica per SM the CTA-per-replica sweep's class chain is shorter."""
+    n, eu, ev, ew = synth.erdos_renyi(200, 0.5, 3)
+    P = IsingProblem(n, eu, ev, np.where(np.arange(ew.size) % 2, 90, -ew).astype(np.int32))
+    s = P.scaled_schedule(20, 2)
+    before = sweep_launches(kernel)
+    r = P.solve(s, R, 3)
+    assert sweep_launches(kernel) == before + 1
+    G = O.Graph(n, eu, ev, np.where(np.arange(ew.size) % 2, 90, -ew).astype(np.int32))
+    order, _ = P.colouring()
+    temps = O.temperatures(s.t_hot, s.t_cold, s.anneal_sweeps, s.hold_sweeps)
+    for k in (0, R - 1):
+        key, half = O.ising_key_half(k, 3)
+        x, _, e = G.anneal_coloured(order, temps, key, half=half)
+        assert (r.branches()[k] == x).all() and r.energies_tracked()[k] == e

@@ -10,7 +10,7 @@ import numpy as np
 import pytest
 
 from oracle import oracle as O
-from qublar_b200 import Budget, IsingProblem, solve_batch, synth
+from qublar_b200 import Budget, IsingProblem, solve_batch, sweep_launches, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -114,3 +114,23 @@ def test_whole_device_words_equal_the_field_sweep(n, d, R, monkeypatch):
     assert (r.branches() == o.branches()).all() and (r.fields() == o.fields()).all()
     assert (r.energies_tracked() == o.energies_tracked()).all() and (r.energies() == o.energies()).all()
     assert (r.marginals() == o.marginals()).all()
+
+
+@pytest.mark.parametrize("graph,R,kernel", [("long rows", 200, "ising_fields"), ("long rows", 4096, "ising_word_16"),
+                                            ("short rows", 200, "ising_word_16")])
+def test_words_are_taken_where_their_class_step_pays(graph, R, kernel):
+    """Long rows make the word sweep's class step long: few replicas of such a
+    graph stay on the CTA-per-replica sweep."""
+    g = synth.erdos_renyi(400, 0.5, 4) if graph == "long rows" else synth.random_regular(700, 20, 4)
+    P = IsingProblem(*g)
+    s = P.scaled_schedule(40, 2)
+    before = sweep_launches(kernel)
+    r = P.solve(s, R, 2)
+    assert sweep_launches(kernel) == before + 1
+    G = O.Graph(*g)
+    order, _ = P.colouring()
+    temps = O.temperatures(s.t_hot, s.t_cold, s.anneal_sweeps, s.hold_sweeps)
+    for k in (0, 1, R - 1):
+        key, half = O.ising_key_half(k, 2)
+        x, f, e = G.anneal_coloured(order, temps, key, half=half)
+        assert (r.branches()[k] == x).all() and r.energies_tracked()[k] == e and (r.fields()[k] == f).all()
