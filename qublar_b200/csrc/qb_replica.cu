@@ -30,6 +30,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
+#include <cmath>
 #include <cstdint>
 #include <cstdlib>
 
@@ -430,6 +432,37 @@ double replica_class(const IsingPlan& p) { return double(p.n) / std::max(1, p.co
 constexpr size_t kReplicaSmem = size_t(226) * 1024;
 constexpr double kReplicaMaxT = 0x1.0p40;
 
+// Clusters of `size` CTAs with an SM each that the device runs at once (a cluster
+// stays within one GPC, so fewer than SMs / size), read once per device.
+int cluster_room(int size) {
+    constexpr int kDevices = 64;
+    static std::atomic<int> known[kDevices][4];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev >= kDevices) return 0;
+    std::atomic<int>& room = known[dev][size <= 2 ? 1 : size <= 4 ? 2 : 3];
+    if (const int r = room.load(std::memory_order_relaxed)) return r;
+    auto kern = ising_replica_kernel<int8_t, true>;
+    if (allow_max_smem(kern) != cudaSuccess) return 0;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = unsigned(size);
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(unsigned(size));
+    cfg.blockDim = dim3(32 * kReplicaWarps);
+    cfg.dynamicSmemBytes = kReplicaSmem;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    room.store(n, std::memory_order_relaxed);
+    return n;
+}
+
 // Cycles of a class step, and of a block of 32 draws in one warp (measured;
 // only their ratio matters, for the number of helper CTAs).
 constexpr double kStepCycles = 260.0, kDrawCycles = 1500.0;
@@ -511,12 +544,14 @@ qb_status launch_ising_replicas(const IsingPlan& p, const SolveBuffers& b, int R
     A.ahead = replica_ahead(p);
     // helper CTAs where SMs are idle, as many as keep the drawing (about
     // kDrawCycles per 32 draws and warp) below the class steps; without them
-    // the CTA's other warps draw
+    // the CTA's other warps draw. Only clusters that all run at once: 16 clusters
+    // of 8 do not, and a second wave doubles the time (4,096 bits of a torus, 16
+    // replicas x 40 sweeps: 0.36 ms, 0.19 for one replica)
     auto drawing = [&](int warps) { return kDrawCycles * std::ceil(double(A.ahead) * blocks / warps) / A.ahead; };
     const double steps = kStepCycles * A.n_colours;
     A.cluster = 1;
     if (drawing(kReplicaWarps - A.consumers) > steps)
-        while (A.cluster < 8 && R * A.cluster * 2 <= word_sms() &&
+        while (A.cluster < 8 && R * A.cluster * 2 <= word_sms() && R <= cluster_room(2 * A.cluster) &&
                (A.cluster == 1 || drawing(kReplicaWarps * (A.cluster - 1)) > steps))
             A.cluster *= 2;
     A.producers = A.cluster > 1 ? kReplicaWarps - A.consumers : std::min(kReplicaWarps - A.consumers, A.ahead * blocks);

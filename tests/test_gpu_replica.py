@@ -90,3 +90,20 @@ def test_dense_graphs_leave_the_dense_kernel_where_its_waves_are_longer(R, kerne
         key, half = O.ising_key_half(k, 3)
         x, _, e = G.anneal_coloured(order, temps, key, half=half)
         assert (r.branches()[k] == x).all() and r.energies_tracked()[k] == e
+
+
+def test_replicas_with_helper_ctas_run_in_one_wave():
+    """Sixteen clusters of eight CTAs do not fit the device at once: a second
+    wave of clusters would double the time of eight replicas."""
+    P = IsingProblem(*_sparse(4001, 8000, 1, 4))
+    s = P.scaled_schedule(300, 0)
+    ms, before = {}, sweep_launches("ising_replica_w8")
+    for R in (8, 16):
+        t = []
+        for _ in range(5):
+            r = P.solve(s, R, 0)
+            t.append(r.info().anneal_ms)
+            r.close()
+        ms[R] = min(t)
+    assert sweep_launches("ising_replica_w8") == before + 10
+    assert ms[16] < 1.5 * ms[8], ms
