@@ -34,7 +34,9 @@ qb_status launch_ising_anneal(const IsingPlan& p, const SolveBuffers& b, int R, 
 // At most one replica per SM, or a dense graph of any number: the sweeps with
 // the draws off their chain (qb_replica.cu); t_max: the schedule's largest
 // temperature. dense_solve_us: the estimated time of a dense graph's solve.
+// replica_csr_fit: whether the few-replica sweep has the adjacency on chip.
 double dense_solve_us(const IsingPlan& p, int R, int sweeps);
+bool replica_csr_fit(const IsingPlan& p);
 bool replica_solve_fit(const IsingPlan& p, int R, double t_max);
 qb_status launch_ising_replicas(const IsingPlan& p, const SolveBuffers& b, int R, int sweeps, uint64_t seed0,
                                 cudaStream_t st);

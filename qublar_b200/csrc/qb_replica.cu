@@ -429,6 +429,20 @@ size_t replica_base_smem(const IsingPlan& p) {
 }
 size_t replica_csr_smem(const IsingPlan& p) { return size_t(p.nnz) * size_t(2 + p.weight_bytes); }
 double replica_class(const IsingPlan& p) { return double(p.n) / std::max(1, p.col.n_colours()); }
+// Consumer warps: a few bits of an average class each, so that the flips' rows
+// are spread (ER(800, 0.06): 9.5 ms at 2 warps, 8.6 at 8, 9.1 at 16).
+int replica_log2_consumers(const IsingPlan& p) {
+    int l = 0;
+    while (l < 4 && replica_class(p) > 6.0 * (1 << l)) ++l;
+    return l;
+}
+// A warp per accepted flip while few of a warp's lanes can flip and rows are
+// long (ER(800, 0.06): 8.6 ms against 20 with a lane per flip; 3,001 bits of
+// degree 8: 2.4 ms against 1.8).
+bool replica_coop(const IsingPlan& p) {
+    const double per = std::ceil(replica_class(p) / (1 << replica_log2_consumers(p)));
+    return 1.5 * per * ((p.max_deg + 31) / 32) < double(p.nnz) / p.n;
+}
 constexpr size_t kReplicaSmem = size_t(226) * 1024;
 constexpr double kReplicaMaxT = 0x1.0p40;
 
@@ -469,6 +483,8 @@ constexpr double kStepCycles = 260.0, kDrawCycles = 1500.0;
 
 }  // namespace
 
+bool replica_csr_fit(const IsingPlan& p) { return replica_base_smem(p) + replica_csr_smem(p) <= kReplicaSmem; }
+
 double dense_solve_us(const IsingPlan& p, int R, int sweeps) {
     // a visit takes 50, 65 or 95 ns by its registers; CTAs of an SM share it
     // from about nine on. 200 bits, 20 sweeps: 0.39 ms for 148 replicas, 1.91
@@ -482,16 +498,21 @@ double dense_solve_us(const IsingPlan& p, int R, int sweeps) {
 
 // One wave of replicas (one CTA per SM) with the state in shared memory, or a
 // dense graph. With the CSR in global memory only classes of at most a few
-// hundred bits gain (n = 2000, degree 50, 100 replicas x 200 sweeps: 2.7 ms
-// against 3.5 for the CTA-per-replica sweep; n = 10,000, degree 40, classes of
-// 600: 17.5 against 14.7). QB_ISING_THREADS asks for that sweep's CTA size,
-// hence for that sweep.
+// hundred bits with a warp per flip and rows of up to 128 gain (2,000 bits of
+// degree 120, 16 replicas x 50 sweeps: 1.82 ms against 2.15 for the
+// CTA-per-replica sweep; ER(800, 0.5) 7.07 against 4.89; 10,000 bits of degree
+// 40, classes of 600, 17.5 against 14.7). Where no SM is left for helper CTAs, wide classes
+// of a small graph wait for the draws (1,600 bits in 2 classes, 148 replicas:
+// 0.179 against 0.167; 4,225 in 4: 0.39 against 0.44). QB_ISING_THREADS asks for
+// that sweep's CTA size, hence for that sweep.
 bool replica_solve_fit(const IsingPlan& p, int R, double t_max) {
     if (t_max > kReplicaMaxT || std::getenv("QB_ISING_THREADS")) return false;
     if (dense_fit(p)) return true;
-    const size_t base = replica_base_smem(p);
-    return R <= word_sms() && base <= kReplicaSmem &&
-           (base + replica_csr_smem(p) <= kReplicaSmem || replica_class(p) <= 300.0);
+    if (R > word_sms() || replica_base_smem(p) > kReplicaSmem) return false;
+    const bool helpers = 2 * R <= word_sms() && R <= cluster_room(2);
+    if (!helpers && replica_class(p) > 300.0 && p.n < (p.weight_bytes == 1 ? 4200 : 6000)) return false;
+    if (replica_csr_fit(p)) return true;
+    return replica_class(p) <= 300.0 && p.nnz <= 128 * int64_t(p.n) && replica_coop(p);
 }
 
 qb_status launch_ising_replicas(const IsingPlan& p, const SolveBuffers& b, int R, int sweeps, uint64_t seed0,
@@ -527,19 +548,9 @@ qb_status launch_ising_replicas(const IsingPlan& p, const SolveBuffers& b, int R
         count_sweep(Sweep::kIsingDense);
         return QB_OK;
     }
-    // consumer warps: a few bits of an average class each, so that the flips'
-    // rows are spread (ER(800, 0.06): 9.5 ms at 2 warps, 8.6 at 8, 9.1 at 16)
-    const double avg = replica_class(p);
-    A.consumers = 1;
-    while (A.consumers < 16 && avg > 6.0 * A.consumers) {
-        A.consumers *= 2;
-        ++A.log2c;
-    }
-    // a warp per accepted flip while few of a warp's lanes can flip and rows are
-    // long (ER(800, 0.06): 8.6 ms against 20 with a lane per flip; 3,001 bits of
-    // degree 8: 2.4 ms against 1.8)
-    const double per = std::ceil(avg / A.consumers);
-    A.coop = 1.5 * per * ((p.max_deg + 31) / 32) < double(p.nnz) / p.n ? 1 : 0;
+    A.log2c = replica_log2_consumers(p);
+    A.consumers = 1 << A.log2c;
+    A.coop = replica_coop(p) ? 1 : 0;
     const int blocks = (p.n + 31) / 32;
     A.ahead = replica_ahead(p);
     // helper CTAs where SMs are idle, as many as keep the drawing (about
@@ -555,7 +566,7 @@ qb_status launch_ising_replicas(const IsingPlan& p, const SolveBuffers& b, int R
                (A.cluster == 1 || drawing(kReplicaWarps * (A.cluster - 1)) > steps))
             A.cluster *= 2;
     A.producers = A.cluster > 1 ? kReplicaWarps - A.consumers : std::min(kReplicaWarps - A.consumers, A.ahead * blocks);
-    const bool csr = replica_base_smem(p) + replica_csr_smem(p) <= kReplicaSmem;
+    const bool csr = replica_csr_fit(p);
     const size_t smem = replica_base_smem(p) + (csr ? replica_csr_smem(p) : 0);
     void (*kern)(ReplicaArgs) = p.weight_bytes == 1 ? (csr ? ising_replica_kernel<int8_t, true> : ising_replica_kernel<int8_t, false>)
                                                     : (csr ? ising_replica_kernel<int32_t, true> : ising_replica_kernel<int32_t, false>);

@@ -107,3 +107,22 @@ def test_replicas_with_helper_ctas_run_in_one_wave():
         ms[R] = min(t)
     assert sweep_launches("ising_replica_w8") == before + 10
     assert ms[16] < 1.5 * ms[8], ms
+
+
+@pytest.mark.parametrize("make,R,kernel", [
+    (lambda: synth.erdos_renyi(500, 0.6, 3), 5, "ising_fields"),            # rows of 300, adjacency off chip
+    (lambda: synth.random_regular(2000, 100, 3), 5, "ising_replica_w8_far"),
+    (lambda: _sparse(2001, 9000, 100, 6), 100, "ising_fields"),             # wide classes, no SM for helpers
+    (lambda: _sparse(2001, 9000, 100, 6), 60, "ising_replica_w8"),
+    (lambda: _sparse(6001, 9000, 900, 6), 100, "ising_replica_w32"),
+])
+def test_the_few_replica_sweep_is_taken_where_it_pays(make, R, kernel, monkeypatch):
+    P = IsingProblem(*make())
+    s = P.scaled_schedule(12, 1)
+    before = sweep_launches(kernel)
+    r = P.solve(s, R, 4)
+    assert sweep_launches(kernel) == before + 1
+    monkeypatch.setenv("QB_ISING_THREADS", "256")
+    o = P.solve(s, R, 4)
+    assert (r.branches() == o.branches()).all() and (r.fields() == o.fields()).all()
+    assert (r.energies_tracked() == o.energies_tracked()).all()
