@@ -847,9 +847,8 @@ qb_status launch_word_solve(const IsingPlan& p, uint8_t* x, int32_t* f, long lon
                               reinterpret_cast<const WordBundle*>(base + kCtl + ib), reinterpret_cast<int*>(base), st);
 }
 
-// Large graphs of few classes: a class step of the whole device costs about 2.7
-// us, a sweep of the CTA-per-replica kernels about 2.3 ns a bit (26,000 bits, 5
-// classes: 60 us against 14).
+// Large graphs of few classes, whose class steps can be worth a grid barrier
+// (ising_route weighs it against a CTA per replica).
 // The barrier's counter holds 2^32 arrivals, the pass index 2^31.
 bool word_grid_fit(const IsingPlan& p, int R, int sweeps) {
     return word_sweep(p) && int64_t(p.n) * ((R + 31) / 32) < (int64_t(1) << 30) &&

@@ -134,3 +134,19 @@ def test_words_are_taken_where_their_class_step_pays(graph, R, kernel):
         key, half = O.ising_key_half(k, 2)
         x, f, e = G.anneal_coloured(order, temps, key, half=half)
         assert (r.branches()[k] == x).all() and r.energies_tracked()[k] == e and (r.fields()[k] == f).all()
+
+
+@pytest.mark.parametrize("L,R,kernel", [(64, 16, "ising_replica_w8"), (64, 148, "ising_fields"), (100, 16, "ising_grid_16"),
+                                        (128, 100, "ising_grid_16")])
+def test_the_whole_device_is_taken_where_its_class_step_pays(L, R, kernel, monkeypatch):
+    """Two classes of L x L / 2 bits: a grid barrier costs more than a CTA's visit
+    of 2,048 of them and less than one of 5,000."""
+    P = IsingProblem(*synth.torus_pm1(L, 5))
+    s = P.scaled_schedule(20, 2)
+    before = sweep_launches(kernel)
+    r = P.solve(s, R, 2)
+    assert sweep_launches(kernel) == before + 1
+    monkeypatch.setenv("QB_ISING_THREADS", "512")
+    o = P.solve(s, R, 2)
+    assert (r.branches() == o.branches()).all() and (r.fields() == o.fields()).all()
+    assert (r.energies_tracked() == o.energies_tracked()).all()
