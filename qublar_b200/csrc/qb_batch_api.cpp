@@ -191,6 +191,37 @@ struct Work {
     WordWork words;
 };
 
+// An instance's groups on the packed kernel at shape `c`: the next group of r
+// remaining replicas, and whether its state runs in place on global memory.
+int field_group(const qb_batch_config& c, int n, int r, bool* global) {
+    const int widest = std::min(c.max_group, floor_pow2(r));
+    int G = widest;
+    while (G > 1 && batch_item_smem(n, G) > size_t(c.smem_bytes)) G /= 2;
+    *global = batch_item_smem(n, G) > size_t(c.smem_bytes);
+    return *global ? widest : G;   // in global memory a wide group keeps the state accesses coalesced
+}
+int field_items(const qb_batch_config& c, int n, int R) {
+    int items = 0;
+    bool global;
+    for (int r0 = 0; r0 < R; r0 += field_group(c, n, R - r0, &global)) ++items;
+    return items;
+}
+
+// Whether an instance of wide classes sweeps faster with one or two replicas to
+// a CTA on the packed kernel than as a word unit of four, given an SM for each:
+// 1.1 + 0.18 deg ns a bit with one, 1.2 + 0.29 deg with two, 2.7 a bit and 16
+// neighbours in a word unit (40 sweeps of one instance, 32 replicas, packed and
+// words: 12,000 bits of degree 5 0.85 and 1.30 ms, 15,000 of degree 20 2.62 and
+// 3.24, 9,900 of degree 40 3.35 and 2.79, 5,000 of degree 3 0.48 and 0.55,
+// 4,000 of degree 5, four to a CTA, 0.77 and 0.47).
+bool spread_pays(const qb_batch_config& c, const IsingPlan& P, int R) {
+    bool global;
+    const int G = field_group(c, P.n, R, &global);
+    if (global || G > 2 || c.threads < 512 || P.n < 512 * P.col.n_colours()) return false;
+    const double deg = double(P.nnz) / P.n;
+    return (G == 1 ? 1.1 + 0.18 * deg : 1.2 + 0.29 * deg) < 2.7 * std::max(1.0, std::ceil(deg / 16.0));
+}
+
 // Splits every instance into replica groups for the shape `c`, sorts the
 // units largest first and writes their descriptors. words: whether instances may
 // run as word units; bound: the smem_bytes that the caller gave (0: none).
@@ -201,6 +232,18 @@ qb_status build_items(qb_batch* b, const qb_batch_config& c, bool words, int bou
                       const double* sample_temp, Work& work) {
     std::vector<IsingItem>& out = work.items;
     const size_t word_cap = word_max_smem();
+    // a batch that leaves SMs idle spreads its large instances over them (only
+    // if all its word instances gain: two launches run one after the other)
+    if (words) {
+        int64_t items = 0;
+        bool spread = true;
+        for (const qb_batch::Inst& I : b->inst) {
+            items += field_items(c, I.n, I.R);
+            if (batch_as_words(I.prob->ising, I.R, bound, word_cap)) spread &= spread_pays(c, I.prob->ising, I.R);
+            if (!spread || items > word_sms()) break;
+        }
+        if (spread && items <= word_sms()) words = false;
+    }
     auto as_words = [&](const qb_batch::Inst& I) {
         return words && batch_as_words(I.prob->ising, I.R, bound, word_cap);
     };
@@ -237,11 +280,8 @@ qb_status build_items(qb_batch* b, const qb_batch_config& c, bool words, int bou
         }
         int r0 = 0;
         while (r0 < I.R) {
-            const int G0 = std::min(c.max_group, floor_pow2(I.R - r0));
-            int G = G0;
-            while (G > 1 && batch_item_smem(I.n, G) > size_t(c.smem_bytes)) G /= 2;
-            const bool global = batch_item_smem(I.n, G) > size_t(c.smem_bytes);
-            if (global) G = G0;   // in global memory a wide group keeps the state accesses coalesced
+            bool global;
+            const int G = field_group(c, I.n, I.R - r0, &global);
             Unit u{int(k), r0, G, global, 0, 0.0};
             if (global) {
                 u.state_off = state_bytes;

@@ -169,3 +169,20 @@ def test_autotune_times_what_its_shape_concerns():
     D = solve_batch(items)
     for k in range(2):
         assert (B.branches(k) == D.branches(k)).all() and (B.energies_tracked(k) == D.energies_tracked(k)).all()
+
+
+@pytest.mark.parametrize("n,d,R,count,packed", [(12000, 5, 5, 2, True), (5001, 3, 9, 1, True), (12000, 5, 32, 5, False),
+                                                (9900, 12, 4, 1, False), (20001, 5, 4, 1, False), (4000, 5, 8, 1, False)])
+def test_few_large_instances_spread_over_the_device(n, d, R, count, packed):
+    """While SMs are idle, large instances of short rows run one or two replicas
+    to a CTA on the packed kernel, otherwise as words; the same results."""
+    probs = [IsingProblem(*synth.random_regular(n, d, 7 + k)) for k in range(count)]
+    sched = probs[0].scaled_schedule(8, 1)
+    before = sweep_launches("ising_batch"), sweep_launches("ising_word_16")
+    B = solve_batch([(P, sched, R, 4 * k) for k, P in enumerate(probs)])
+    assert (sweep_launches("ising_batch") - before[0], sweep_launches("ising_word_16") - before[1]) == \
+        ((1, 0) if packed else (0, 1))
+    for k, P in enumerate(probs):
+        r = P.solve(sched, R, 4 * k)
+        assert (B.branches(k) == r.branches()).all() and (B.energies_tracked(k) == r.energies_tracked()).all()
+        assert (B.marginals(k) == r.marginals()).all()
