@@ -449,8 +449,9 @@ typedef struct qb_server_config {
                                     (0 = no limit) */
     int32_t coop_parts;          /* cooperative sweeps (lockstep residual, weighted QUBO) run side by side, up
                                     to this many at once, each on a grid sized to its problem (at most half the
-                                    device; the grids together within what the device holds at once)
-                                    (0 = 4; 1 = each alone on the whole device) */
+                                    device; the grids together within what the device holds at once); problems
+                                    whose sweep needs no grid run beside them on the residual streams
+                                    (0 = 4; 1 = lockstep residual and QUBO requests each alone on the device) */
 } qb_server_config;
 
 /* Request states reported by qb_server_poll. */

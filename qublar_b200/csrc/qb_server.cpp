@@ -1,9 +1,10 @@
 // The serving loop of the C ABI (qb_server_*): admission by a device-memory
 // budget, ising requests advanced together in ticks of the packed kernel
-// (one CUDA-graph replay per tick, state resident between ticks), residual
-// requests as cluster launches on a stream pool beside the ticks, and the
-// cooperative sweeps (lockstep residual, weighted QUBO) side by side on equal
-// partitions of the device's SMs, one cooperative grid per request.
+// (one CUDA-graph replay per tick, state resident between ticks), requests
+// whose sweep has no grid barrier (cluster and local residual sweeps, small
+// weighted QUBOs) on a stream pool beside the ticks, and the cooperative sweeps
+// (lockstep residual, weighted QUBO) side by side on partitions of the device's
+// SMs, one cooperative grid per request.
 //
 // One worker thread owns every device call of the loop. It never holds the
 // server mutex across a CUDA call that waits, and it polls completion events
@@ -80,10 +81,11 @@ struct Request {
     int64_t charge_work = 0;      // problem + working memory: returned when the request finishes
     int64_t charge_results = 0;   // results: returned when the client releases them
     bool cancel = false;
+    bool in_cta = false;          // its sweep keeps a branch (32 QUBO replicas) in one CTA: no grid barrier, no scratch
     bool coop = false;            // a cooperative sweep (lockstep residual or weighted QUBO)
     bool exclusive = false;       // ... on the whole device, with nothing beside it (no partition plan)
     int part = -1;                // the stream a side-by-side cooperative sweep runs on
-    int ctas = 0;                 // ... and its grid (CTAs taken from the device's cooperative budget)
+    int ctas = 0;                 // SMs taken from the device's cooperative budget: its grid, or its in-CTA sweep's CTAs
     // device memory (stream-ordered allocations)
     DevBuf d_x, d_f, d_e, d_p, d_temp, d_state, d_drift, d_accepts, d_ef64, d_etrack;
     // ising progress
@@ -134,9 +136,11 @@ struct qb_server {
     Request* exclusive_run = nullptr;
     // cooperative sweeps side by side: up to `parts` at once, each on its own
     // stream with a grid sized to its problem, their grids together within the
-    // CTAs the device holds at once (coop_budget), one grid at most coop_cap
+    // CTAs the device holds at once (coop_budget), one grid at most coop_cap. The
+    // in-CTA sweeps' CTAs (cta_used) count against the next grid: a grid that is
+    // admitted finds its SMs free of them, so all of it becomes resident
     int parts = 1;
-    int coop_budget = 0, coop_cap = 0, coop_used = 0;
+    int coop_budget = 0, coop_cap = 0, coop_used = 0, cta_used = 0;
     int full_resid = 0, full_qubo = 0;
     std::vector<cudaStream_t> part_streams;
     std::vector<Request*> part_run;
@@ -197,11 +201,18 @@ int64_t ising_work_bytes(const qb_problem* p, int R, int sweeps) {
     return p->device_bytes + n * R * 5 + int64_t(sweeps) * 8;
 }
 int64_t ising_result_bytes(int n, int R) { return int64_t(n) * R * 5 + int64_t(R) * 8 + int64_t(n) * 4; }
-int64_t resid_work_bytes(const qb_problem* p, int R, int sweeps) {
-    int64_t b = p->device_bytes + int64_t(sweeps) * 8 + int64_t(R) * 12;
-    if (p->kind == QB_KIND_RESIDUAL && p->resid.variant == QB_RESID_LOCKSTEP)
-        b += int64_t(resid_lockstep_scratch(p->resid, std::min(R, resid_lockstep_max_branches())));
-    if (p->kind == QB_KIND_QUBO) b += int64_t(qubo_scratch(p->qubo)) + int64_t(R) * 8;
+// Scratch of a cooperative sweep: its barrier and timeout flag (all an in-CTA
+// sweep keeps of it), and the branches' state.
+size_t coop_scratch(const qb_problem* p, int R, bool in_cta) {
+    if (in_cta) return 64;
+    return p->kind == QB_KIND_QUBO ? qubo_scratch(p->qubo)
+                                   : resid_lockstep_scratch(p->resid, std::min(R, resid_lockstep_max_branches()));
+}
+int64_t resid_work_bytes(const Request* r) {
+    const qb_problem* p = r->prob;
+    int64_t b = p->device_bytes + int64_t(r->sweeps) * 8 + int64_t(r->R) * 12;
+    if (r->coop) b += int64_t(coop_scratch(p, r->R, r->in_cta));
+    if (p->kind == QB_KIND_QUBO) b += int64_t(r->R) * 8;
     return b;
 }
 int64_t resid_result_bytes(int n, int R) { return int64_t(n) * R + int64_t(R) * 8 + int64_t(n) * 4; }
@@ -305,108 +316,104 @@ qb_status admit_ising(qb_server* S, Request* r) {
     return QB_OK;
 }
 
-qb_status launch_resid(qb_server* S, Request* r) {
+// Temperatures and result buffers of a residual or QUBO request on the upload
+// stream; scratch: bytes of d_state, its first 64 zeroed.
+qb_status stage_request(qb_server* S, Request* r, size_t scratch) {
     qb_status s;
-    cudaStream_t st = S->resid_streams[size_t(S->next_resid_stream)];
-    S->next_resid_stream = (S->next_resid_stream + 1) % int(S->resid_streams.size());
-    {
-        AsyncAllocScope scope(S->upload_stream);
-        if ((s = problem_upload(r->prob, S->upload_stream)) != QB_OK) return s;
-        const std::vector<double> temp = temperatures(r->sched);
-        if ((s = upload_vec(r->d_temp, temp, S->upload_stream))) return s;
-        if ((s = r->d_x.alloc(size_t(r->R) * size_t(r->n)))) return s;
-        if ((s = r->d_drift.alloc(size_t(r->R) * 4))) return s;
-        if ((s = r->d_accepts.alloc(size_t(r->R) * 8))) return s;
-        if ((s = r->d_ef64.alloc(size_t(r->R) * 8))) return s;
-        if ((s = r->d_p.alloc(size_t(r->n) * 4))) return s;
-        QB_CUDA(cudaMemsetAsync(r->d_drift.p, 0, r->d_drift.bytes, S->upload_stream));
-        QB_CUDA(cudaMemsetAsync(r->d_accepts.p, 0, r->d_accepts.bytes, S->upload_stream));
-        QB_CUDA(cudaStreamSynchronize(S->upload_stream));   // `temp` is a local
-    }
-    const ResidualPlan& P = r->prob->resid;
+    const bool qubo = r->kind == QB_KIND_QUBO;
+    AsyncAllocScope scope(S->upload_stream);
+    if ((s = problem_upload(r->prob, S->upload_stream)) != QB_OK) return s;
+    const std::vector<double> temp = temperatures(r->sched);
+    if ((s = upload_vec(r->d_temp, temp, S->upload_stream))) return s;
+    if ((s = r->d_state.alloc(scratch))) return s;
+    if ((s = r->d_x.alloc(size_t(r->R) * size_t(r->n)))) return s;
+    if ((s = r->d_drift.alloc(size_t(r->R) * 4))) return s;
+    if ((s = r->d_accepts.alloc(size_t(r->R) * 8))) return s;
+    if ((s = r->d_ef64.alloc(size_t(r->R) * 8))) return s;
+    if ((s = r->d_p.alloc(size_t(r->n) * 4))) return s;
+    if (qubo && (s = r->d_etrack.alloc(size_t(r->R) * 8))) return s;
+    QB_CUDA(cudaMemsetAsync(r->d_drift.p, 0, r->d_drift.bytes, S->upload_stream));
+    QB_CUDA(cudaMemsetAsync(r->d_accepts.p, 0, r->d_accepts.bytes, S->upload_stream));
+    if (qubo) QB_CUDA(cudaMemsetAsync(r->d_etrack.p, 0, r->d_etrack.bytes, S->upload_stream));
+    if (scratch) QB_CUDA(cudaMemsetAsync(r->d_state.p, 0, 64, S->upload_stream));   // barrier counter and timeout flag
+    QB_CUDA(cudaStreamSynchronize(S->upload_stream));   // `temp` is a local
+    return QB_OK;
+}
+
+SolveBuffers resid_buffers(Request* r, int b0) {
     SolveBuffers b;
-    b.x = r->d_x.as<uint8_t>();
+    b.x = r->d_x.as<uint8_t>() + size_t(b0) * size_t(r->n);
     b.temp = r->d_temp.as<double>();
-    b.drift = r->d_drift.as<float>();
-    b.accepts = r->d_accepts.as<unsigned long long>();
-    b.e_f64 = r->d_ef64.as<double>();
-    b.p = r->d_p.as<float>();
-    if (resid_local_route(P, r->R)) s = launch_resid_local(P, b, r->R, r->sweeps, r->sched.refresh_sweeps, r->seed0, st);
-    else s = launch_resid_anneal(P, b, r->R, r->sweeps, r->sched.refresh_sweeps, r->seed0, st);
+    b.drift = r->d_drift.as<float>() + b0;
+    b.accepts = r->d_accepts.as<unsigned long long>() + b0;
+    b.scratch = r->d_state.p;
+    return b;
+}
+
+QuboBuffers qubo_buffers(Request* r, int b0) {
+    QuboBuffers b;
+    b.x = r->d_x.as<uint8_t>() + size_t(b0) * size_t(r->n);
+    b.temp = r->d_temp.as<double>();
+    b.drift = r->d_drift.as<float>() + b0;
+    b.e_track = r->d_etrack.as<double>() + b0;
+    b.accepts = r->d_accepts.as<unsigned long long>() + b0;
+    b.scratch = r->d_state.p;
+    return b;
+}
+
+// The whole schedule of a request whose sweep has no grid barrier.
+qb_status launch_in_cta(Request* r, cudaStream_t st) {
+    if (r->kind == QB_KIND_QUBO)
+        return launch_qubo_small(r->prob->qubo, qubo_buffers(r, 0), r->R, r->sweeps, r->sched.refresh_sweeps, r->seed0, st);
+    return launch_resid_local(r->prob->resid, resid_buffers(r, 0), r->R, r->sweeps, r->sched.refresh_sweeps, r->seed0, st);
+}
+
+// Energies and marginals of the finished branches, and the event behind them.
+qb_status launch_results(Request* r, cudaStream_t st) {
+    qb_status s;
+    const uint8_t* x = r->d_x.as<uint8_t>();
+    if (r->kind == QB_KIND_QUBO) s = launch_qubo_energies(r->prob->qubo, x, r->R, r->d_ef64.as<double>(), st);
+    else s = launch_resid_energies(r->prob->resid, x, r->R, r->d_ef64.as<double>(), st);
     if (s != QB_OK) return s;
-    if ((s = launch_resid_energies(P, b.x, r->R, b.e_f64, st))) return s;
-    if ((s = launch_marginals(b.x, r->R, r->n, b.p, st))) return s;
+    if ((s = launch_marginals(x, r->R, r->n, r->d_p.as<float>(), st))) return s;
     QB_CUDA(cudaEventCreateWithFlags(&r->done_ev, cudaEventDisableTiming));
     QB_CUDA(cudaEventRecord(r->done_ev, st));
     return QB_OK;
 }
 
-// A cooperative sweep (lockstep residual or weighted QUBO) on stream `st`:
-// the whole device (exclusive requests) or one partition's grid; its scratch
-// lives in d_state.
-qb_status launch_coop(qb_server* S, Request* r, cudaStream_t st, int qubo_ctas) {
+// A request beside the ticks on the stream pool: an in-CTA sweep or the cluster sweep.
+qb_status launch_resid(qb_server* S, Request* r) {
     qb_status s;
-    const bool qubo = r->kind == QB_KIND_QUBO;
-    {
-        AsyncAllocScope scope(S->upload_stream);
-        if ((s = problem_upload(r->prob, S->upload_stream)) != QB_OK) return s;
-        const std::vector<double> temp = temperatures(r->sched);
-        if ((s = upload_vec(r->d_temp, temp, S->upload_stream))) return s;
-        const size_t scratch = qubo ? qubo_scratch(r->prob->qubo)
-                                    : resid_lockstep_scratch(r->prob->resid, std::min(r->R, resid_lockstep_max_branches()));
-        if ((s = r->d_state.alloc(scratch))) return s;
-        if ((s = r->d_x.alloc(size_t(r->R) * size_t(r->n)))) return s;
-        if ((s = r->d_drift.alloc(size_t(r->R) * 4))) return s;
-        if ((s = r->d_accepts.alloc(size_t(r->R) * 8))) return s;
-        if ((s = r->d_ef64.alloc(size_t(r->R) * 8))) return s;
-        if ((s = r->d_p.alloc(size_t(r->n) * 4))) return s;
-        if (qubo && (s = r->d_etrack.alloc(size_t(r->R) * 8))) return s;
-        QB_CUDA(cudaMemsetAsync(r->d_drift.p, 0, r->d_drift.bytes, S->upload_stream));
-        QB_CUDA(cudaMemsetAsync(r->d_accepts.p, 0, r->d_accepts.bytes, S->upload_stream));
-        if (qubo) QB_CUDA(cudaMemsetAsync(r->d_etrack.p, 0, r->d_etrack.bytes, S->upload_stream));
-        QB_CUDA(cudaMemsetAsync(r->d_state.p, 0, 64, S->upload_stream));   // barrier counter and timeout flag
-        QB_CUDA(cudaStreamSynchronize(S->upload_stream));   // `temp` is a local
-    }
-    uint8_t* x = r->d_x.as<uint8_t>();
-    if (qubo) {
-        const bool small = qubo_small_fit(r->prob->qubo);
-        const int RB = small ? r->R : qubo_max_branches();
-        for (int b0 = 0; b0 < r->R; b0 += RB) {
-            QuboBuffers qb;
-            qb.x = x + size_t(b0) * size_t(r->n);
-            qb.temp = r->d_temp.as<double>();
-            qb.drift = r->d_drift.as<float>() + b0;
-            qb.e_track = r->d_etrack.as<double>() + b0;
-            qb.accepts = r->d_accepts.as<unsigned long long>() + b0;
-            qb.scratch = r->d_state.p;
-            s = small ? launch_qubo_small(r->prob->qubo, qb, r->R, r->sweeps, r->sched.refresh_sweeps, r->seed0, st)
-                      : launch_qubo_lockstep(r->prob->qubo, qb, std::min(RB, r->R - b0), r->sweeps,
-                                             r->sched.refresh_sweeps, r->seed0 + uint64_t(b0), st, qubo_ctas);
-            if (s != QB_OK) return s;
-        }
-        if ((s = launch_qubo_energies(r->prob->qubo, x, r->R, r->d_ef64.as<double>(), st))) return s;
+    cudaStream_t st = S->resid_streams[size_t(S->next_resid_stream)];
+    S->next_resid_stream = (S->next_resid_stream + 1) % int(S->resid_streams.size());
+    if ((s = stage_request(S, r, 0))) return s;
+    if (r->in_cta) s = launch_in_cta(r, st);
+    else s = launch_resid_anneal(r->prob->resid, resid_buffers(r, 0), r->R, r->sweeps, r->sched.refresh_sweeps, r->seed0, st);
+    return s == QB_OK ? launch_results(r, st) : s;
+}
+
+// A cooperative sweep (lockstep residual or weighted QUBO) on stream `st`:
+// the whole device (exclusive requests, whose sweep may be an in-CTA one) or
+// one partition's grid; its scratch lives in d_state.
+qb_status launch_coop(qb_server* S, Request* r, cudaStream_t st, int qubo_ctas) {
+    qb_status s = stage_request(S, r, coop_scratch(r->prob, r->R, r->in_cta));
+    if (s != QB_OK) return s;
+    if (r->in_cta) {
+        if ((s = launch_in_cta(r, st))) return s;
+    } else if (r->kind == QB_KIND_QUBO) {
+        const int RB = qubo_max_branches();
+        for (int b0 = 0; b0 < r->R; b0 += RB)
+            if ((s = launch_qubo_lockstep(r->prob->qubo, qubo_buffers(r, b0), std::min(RB, r->R - b0), r->sweeps,
+                                          r->sched.refresh_sweeps, r->seed0 + uint64_t(b0), st, qubo_ctas)))
+                return s;
     } else {
-        const ResidualPlan& P = r->prob->resid;
-        const bool local = resid_local_route(P, r->R);
-        const int RB = local ? r->R : resid_lockstep_max_branches();
-        for (int b0 = 0; b0 < r->R; b0 += RB) {
-            SolveBuffers b;
-            b.x = x + size_t(b0) * size_t(r->n);
-            b.temp = r->d_temp.as<double>();
-            b.drift = r->d_drift.as<float>() + b0;
-            b.accepts = r->d_accepts.as<unsigned long long>() + b0;
-            b.scratch = r->d_state.p;
-            if (local) s = launch_resid_local(P, b, r->R, r->sweeps, r->sched.refresh_sweeps, r->seed0, st);
-            else s = launch_resid_lockstep(P, b, std::min(RB, r->R - b0), r->sweeps, r->sched.refresh_sweeps,
-                                           r->seed0 + uint64_t(b0), st);
-            if (s != QB_OK) return s;
-        }
-        if ((s = launch_resid_energies(P, x, r->R, r->d_ef64.as<double>(), st))) return s;
+        const int RB = resid_lockstep_max_branches();
+        for (int b0 = 0; b0 < r->R; b0 += RB)
+            if ((s = launch_resid_lockstep(r->prob->resid, resid_buffers(r, b0), std::min(RB, r->R - b0), r->sweeps,
+                                           r->sched.refresh_sweeps, r->seed0 + uint64_t(b0), st)))
+                return s;
     }
-    if ((s = launch_marginals(x, r->R, r->n, r->d_p.as<float>(), st))) return s;
-    QB_CUDA(cudaEventCreateWithFlags(&r->done_ev, cudaEventDisableTiming));
-    QB_CUDA(cudaEventRecord(r->done_ev, st));
-    return QB_OK;
+    return launch_results(r, st);
 }
 
 // Admits pending requests in arrival order while the budget and the active
@@ -446,10 +453,11 @@ void admit_pending(qb_server* S) {
                 int slot = -1;
                 for (int k = 0; k < int(S->part_run.size()) && slot < 0; ++k)
                     if (!S->part_run[size_t(k)]) slot = k;
-                if (slot < 0 || S->coop_used + q->ctas > S->coop_budget) return;
+                if (slot < 0 || S->coop_used + S->cta_used + q->ctas > S->coop_budget) return;
                 q->part = slot;
                 S->coop_used += q->ctas;
             }
+            if (q->in_cta && !q->coop) S->cta_used += q->ctas;
             S->pending.pop_front();
             S->bytes_in_use += need;
             S->peak_bytes = std::max(S->peak_bytes, S->bytes_in_use);
@@ -468,6 +476,7 @@ void admit_pending(qb_server* S) {
         if (s != QB_OK) {
             const std::string msg = qb_last_error();
             if (r->coop && !r->exclusive) S->coop_used -= r->ctas;   // its grid never ran
+            if (r->in_cta && !r->coop) S->cta_used -= r->ctas;
             drop_work(S, r);
             drop_results(r);
             std::lock_guard<std::mutex> lk(S->mu);
@@ -663,6 +672,7 @@ void fail_all_running(qb_server* S, qb_status st, const std::string& msg) {
     S->running_ising.clear();
     S->running_resid.clear();
     S->tick_inflight = false;
+    S->cta_used = 0;
     for (Request* r : all) {
         drop_work(S, r);
         drop_results(r);
@@ -722,6 +732,7 @@ void poll_resid(qb_server* S) {
             S->fatal = qb_last_error();
         }
         const bool cancelled = r->cancel;
+        if (r->in_cta) S->cta_used -= r->ctas;
         drop_work(S, r);
         std::lock_guard<std::mutex> lk(S->mu);
         if (e != cudaSuccess || cancelled) {
@@ -934,8 +945,15 @@ extern "C" qb_status qb_server_submit(qb_server* S, qb_problem* p, const qb_sche
         r->kind = p->kind;
         r->R = int(n_branches);
         r->n = p->kind == QB_KIND_ISING ? p->ising.n : p->kind == QB_KIND_QUBO ? p->qubo.n : p->resid.n;
-        r->coop = p->kind == QB_KIND_QUBO || (p->kind == QB_KIND_RESIDUAL && p->resid.variant == QB_RESID_LOCKSTEP);
+        // the sweep is chosen here, for the charge, the admission and the launch
+        // alike. One without a grid barrier needs no partition; with coop_parts =
+        // 1 lockstep pyramids and QUBOs run alone whichever sweep they take
+        r->in_cta = p->kind == QB_KIND_QUBO ? qubo_small_fit(p->qubo)
+                                            : p->kind == QB_KIND_RESIDUAL && resid_local_route(p->resid, r->R);
+        r->coop = (p->kind == QB_KIND_QUBO || (p->kind == QB_KIND_RESIDUAL && p->resid.variant == QB_RESID_LOCKSTEP)) &&
+                  (S->parts == 1 || !r->in_cta);
         r->exclusive = r->coop && S->parts == 1;
+        if (r->in_cta) r->ctas = std::min(S->coop_budget, p->kind == QB_KIND_QUBO ? (r->R + 31) / 32 : r->R);
         if (r->coop && !r->exclusive && p->kind == QB_KIND_QUBO) r->ctas = coop_grid(S, p);
         r->sweeps = sch->anneal_sweeps + sch->hold_sweeps;
         if (r->coop && !r->exclusive && p->kind == QB_KIND_RESIDUAL) {
@@ -963,7 +981,7 @@ extern "C" qb_status qb_server_submit(qb_server* S, qb_problem* p, const qb_sche
             r->charge_work = ising_work_bytes(p, r->R, r->sweeps);
             r->charge_results = ising_result_bytes(r->n, r->R);
         } else {
-            r->charge_work = resid_work_bytes(p, r->R, r->sweeps);
+            r->charge_work = resid_work_bytes(r.get());
             r->charge_results = resid_result_bytes(r->n, r->R);
         }
         r->t_submit = now_s();

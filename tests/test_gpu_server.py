@@ -15,7 +15,7 @@ import pytest
 
 from oracle import oracle as O
 from qublar_b200 import (OPT_DEFER_UPLOAD, OPT_RESID_CLUSTER, IsingProblem, QBError, QuboProblem, ResidualProblem,
-                         Schedule, Server, synth)
+                         Schedule, Server, sweep_launches, synth)
 from qublar_b200._abi import REQ_CANCELLED, REQ_DONE
 
 pytestmark = pytest.mark.gpu
@@ -267,6 +267,39 @@ def test_cooperative_requests_overlap_on_partitions_and_match_alone():
         assert (S.branches(ids[3 + k]) == r.branches()).all(), k
     r = IsingProblem(*g1).solve(si, 16, 20)
     assert (S.branches(ids[5]) == r.branches()).all()
+    S.close()
+
+
+def test_requests_without_a_grid_take_no_partition_and_no_scratch():
+    """Lockstep-planned pyramids whose branch fits one CTA, and small QUBOs, need
+    neither a partition nor the cooperative sweeps' scratch: more of them than
+    coop_parts run at once, and a budget without that scratch admits one."""
+    pyrs = [synth.tomography(synth.small_tomo_params(0.16, 20, seed=k + 1)) for k in range(4)]
+    q = synth.random_qubo(150, 700, 3)
+    sp, sq = Schedule(50.0, 1.0, 2500, 50, 50), Schedule(3.0, 0.05, 9000, 20, 32)
+    P = [ResidualProblem.from_arrays(a, flags=DEFER) for a in pyrs]
+    Q = QuboProblem.from_dict(q, flags=DEFER)
+    local, small = sweep_launches("resid_local"), sweep_launches("qubo_small")
+    S = Server(coop_parts=2)
+    ids = [S.submit(p, sp, 16, k) for k, p in enumerate(P)] + [S.submit(Q, sq, 40, 9)]
+    for i in ids:
+        S.wait(i, 120000)
+    infos = [S.info(i) for i in ids]
+    assert sweep_launches("resid_local") == local + 4 and sweep_launches("qubo_small") == small + 1
+    running = max(sum(b.t_admit <= a.t_admit < b.t_done for b in infos) for a in infos)
+    assert running > 2
+    for k, a in enumerate(pyrs):
+        assert (S.branches(ids[k]) == ResidualProblem.from_arrays(a).solve(sp, 16, k).branches()).all()
+    assert (S.branches(ids[4]) == QuboProblem.from_dict(q).solve(sq, 40, 9).branches()).all()
+    S.close()
+    # device bytes, temperatures, counters and results of 64 branches, nothing more
+    P = ResidualProblem.from_arrays(pyrs[0], flags=DEFER)
+    s = Schedule(50.0, 1.0, 20, 5, 25)
+    need = P.info().device_bytes + 25 * 8 + 64 * 12 + 64 * P.n + 64 * 8 + 4 * P.n
+    S = Server(budget_bytes=need + 64)
+    rid = S.submit(P, s, 64)
+    S.wait(rid, 60000)
+    assert S.info(rid).device_bytes <= need
     S.close()
 
 
