@@ -666,7 +666,11 @@ qb_status launch_tick(qb_server* S) {
     S->tick_inflight = true;
     return QB_OK;
 }
+
 void fail_all_running(qb_server* S, qb_status st, const std::string& msg) {
+    // their kernels may still run (the word units of a tick whose items failed to
+    // launch, the requests on other streams): the buffers go back behind them
+    cudaDeviceSynchronize();
     std::vector<Request*> all(S->running_ising);
     all.insert(all.end(), S->running_resid.begin(), S->running_resid.end());
     S->running_ising.clear();
