@@ -247,9 +247,11 @@ struct ResidualPlan {
     std::vector<int32_t> chunk_ptr;
     std::vector<int32_t> h_nbr_new;   // neighbours as sweep-order indices
     std::vector<uint32_t> h_meta;     // lockstep: per bit 8 words {row start, rays, nbr start, nbrs, lin, q, index, 0}
-    bool local = false;               // lockstep plans: a branch fits one CTA (qb_local.cu)
-    std::vector<uint32_t> l_rec;      // local sweep: 8 words per lane pair, 16 pairs per warp item
+    bool local = false;               // a branch fits one CTA (qb_local.cu)
+    std::vector<uint32_t> l_rec;      // local sweep: 8 words per lane pair (lockstep) or lane group (cluster order)
     std::vector<int32_t> l_ptr;       // its warp items per class
+    double l_tail = 0.0;              // cluster order: over the classes, the longest bit's rays beyond 256
+    double l_long = 0.0;              // ... and beyond 1,000
     DevBuf d_lrec, d_lptr;
     // host copies of the sweep-order arrays (h_ent is released after upload)
     std::vector<int32_t> h_row, h_nbr_ptr;

@@ -29,6 +29,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
@@ -412,8 +413,9 @@ static void group_plan(ResidualPlan& P) {
         ++items;
         P.l_rec.resize(size_t(items) * kGroupRecs * 8, 0u);
     };
+    P.l_tail = P.l_long = 0.0;
     for (int c = 0; c < P.col.n_colours(); ++c) {
-        int at = kGroupRecs;
+        int at = kGroupRecs, most = 0;
         for (int k = P.col.class_ptr[size_t(c)]; k < P.col.class_ptr[size_t(c) + 1]; ++k)
             if (P.h_row[size_t(k) + 1] - P.h_row[size_t(k)] > kHeavyRays) {
                 open_item();
@@ -427,6 +429,10 @@ static void group_plan(ResidualPlan& P) {
             }
             put(k, at++, false);
         }
+        for (int k = P.col.class_ptr[size_t(c)]; k < P.col.class_ptr[size_t(c) + 1]; ++k)
+            most = std::max(most, P.h_row[size_t(k) + 1] - P.h_row[size_t(k)]);
+        P.l_tail += std::max(0, most - 32 * kHold);
+        P.l_long += std::max(0, most - 1000);
         P.l_ptr.push_back(items);
     }
 }
@@ -488,11 +494,15 @@ void resid_local_plan(ResidualPlan& P) {
     }
 }
 
-// Microseconds per sweep, fitted to B200 times at 500 to 90,000 bits: a class
+// Microseconds per sweep, fitted to B200 times at 16 to 90,000 bits: a class
 // step of the local sweep costs 1.05 or, once its items outnumber the warps,
 // 0.1 per item; the lockstep sweep 3.9 per class at 16 branches and 13 % more
 // per further 16 (90,000 bits: 16 branches 1.09 ms local, 0.88 lockstep; 64
-// branches 1.09 and 1.22; 40,000 bits, 64 branches 0.54 and 0.83).
+// branches 1.09 and 1.22; 40,000 bits, 64 branches 0.54 and 0.83). Against the
+// cluster sweep, in its order: a warp goes over a bit's rays beyond 256 and its
+// neighbours beyond eight one load behind the other (100 bits of 1,000 rays, 16
+// branches x 45 sweeps 28.0 ms local, 12.9 cluster; 1,000 bits of 48 neighbours,
+// 149 branches 6.5 and 5.0), and a cluster CTA shares its SM with another.
 bool resid_local_route(const ResidualPlan& p, int R) {
     if (!p.local || std::getenv("QB_PHASE_TIMES") || std::getenv("QB_TEST_BARRIER_STALL")) return false;
     const char* k = std::getenv("QB_RESID_KERNEL");
@@ -502,8 +512,12 @@ bool resid_local_route(const ResidualPlan& p, int R) {
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const double classes = p.col.n_colours(), items = p.l_ptr.empty() ? 0.0 : p.l_ptr.back();
     const double local = std::max(1.05 * classes, 0.1 * items) * ((R + sms - 1) / sms);
-    // the cluster sweep: 3.3 a class step (5,000 bits, 18 branches, one CTA a branch)
-    if (p.variant == QB_RESID_CLUSTER) return std::max(1.05 * classes, 0.1 * items) < 3.3 * classes;
+    if (p.variant == QB_RESID_CLUSTER) {
+        const double nbrs = 0.2 * std::max(0.0, double(p.n_nbr) / p.n / 8.0 - 1.0);
+        const double one = std::max((1.05 + nbrs) * classes + 0.0069 * p.l_tail, 0.1 * items) * ((R + sms - 1) / sms);
+        const double load = p.CL == 1 ? std::ceil(R / (2.0 * sms)) : std::max(1.0, R * p.CL / 100.0);
+        return one < (3.3 * classes + 0.0035 * p.l_long) * load;
+    }
     double lock = 0.0;
     for (int left = R; left > 0; left -= resid_lockstep_max_branches()) {
         const int groups = (std::min(left, resid_lockstep_max_branches()) + 15) / 16;

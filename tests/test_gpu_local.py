@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from oracle import oracle as O
-from qublar_b200 import OPT_RESID_CLUSTER, ResidualProblem, Schedule, synth
+from qublar_b200 import OPT_RESID_CLUSTER, ResidualProblem, Schedule, sweep_launches, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -70,3 +70,19 @@ def test_equals_the_planned_sweep_and_the_oracle(name, order, monkeypatch):
     for k in (0, R - 1):
         x, _ = O.resid_anneal_coloured(arr, visits, temps, s.refresh_sweeps, k + 4, mode=P.info().variant)
         assert (X[k] == x).all(), k
+
+
+@pytest.mark.parametrize("make,R,kernel", [
+    (lambda: _random(40, 1200, [1000], 3, 0), 16, "resid_cluster"),          # a warp would walk 1,000 rays
+    (lambda: _random(400, 900, [2], 3, 24), 149, "resid_cluster"),           # 48 neighbours, two waves of branches
+    (lambda: _random(400, 900, [2], 3, 24), 16, "resid_local_cluster"),
+    (lambda: _random(60, 300, [20], 3), 16, "resid_local_cluster"),
+])
+def test_cluster_plans_take_the_local_sweep_where_it_pays(make, R, kernel, monkeypatch):
+    P = ResidualProblem.from_arrays(make(), flags=OPT_RESID_CLUSTER)
+    s = Schedule(20.0, 0.6, 20, 2, 7)
+    before = sweep_launches(kernel)
+    r = P.solve(s, R, 3)
+    assert sweep_launches(kernel) == before + 1
+    monkeypatch.setenv("QB_RESID_KERNEL", "cluster" if "local" in kernel else "local")
+    assert (P.solve(s, R, 3).branches() == r.branches()).all()
