@@ -508,6 +508,9 @@ bool resid_local_route(const ResidualPlan& p, int R) {
     const char* k = std::getenv("QB_RESID_KERNEL");
     if (k && (std::strcmp(k, "lockstep") == 0 || std::strcmp(k, "cluster") == 0)) return false;
     if (k && std::strcmp(k, "local") == 0) return true;
+    // a forced cluster size asks for the cluster sweep
+    const char* cl = std::getenv("QB_RESID_CLUSTER");
+    if (p.variant == QB_RESID_CLUSTER && cl && *cl) return false;
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const double classes = p.col.n_colours(), items = p.l_ptr.empty() ? 0.0 : p.l_ptr.back();

@@ -86,3 +86,14 @@ def test_cluster_plans_take_the_local_sweep_where_it_pays(make, R, kernel, monke
     assert sweep_launches(kernel) == before + 1
     monkeypatch.setenv("QB_RESID_KERNEL", "cluster" if "local" in kernel else "local")
     assert (P.solve(s, R, 3).branches() == r.branches()).all()
+
+
+def test_a_forced_cluster_size_is_the_cluster_sweep(monkeypatch):
+    monkeypatch.setenv("QB_RESID_CLUSTER", "4")
+    P = ResidualProblem.from_arrays(_random(60, 300, [20], 3), flags=OPT_RESID_CLUSTER)
+    s = Schedule(20.0, 0.6, 20, 2, 7)
+    before = sweep_launches("resid_cluster")
+    x = P.solve(s, 5, 3).branches()
+    assert sweep_launches("resid_cluster") == before + 1
+    monkeypatch.delenv("QB_RESID_CLUSTER")
+    assert (P.solve(s, 5, 3).branches() == x).all()
