@@ -89,7 +89,9 @@ __device__ __forceinline__ bool accept_int(uint64_t u53, int k, double T) {
 // 2^-21 + X 2^-20, floor(X) is proven; otherwise the fp64 test of the nearest
 // integer decides. X <= 36.8 T, so the margin stays below 0.17 for T <= 4096;
 // above that X is taken in fp64 (error below (X + T) 2^-45, also the fp64
-// test's own rounding) with the same structure. A zero draw searches.
+// test's own rounding) with the same structure; its last fallback, a margin above
+// 1/4, is beyond the route's limit T <= 2^40 (X <= bound + 1 < 2^32: the margin
+// stays below 2^-4). A zero draw searches.
 __device__ __noinline__ int draw_limit_search(uint64_t u53, double T, int bound) {
     int lo = 0, hi = bound;   // accepted at lo
     while (lo < hi) {

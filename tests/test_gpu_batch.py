@@ -24,6 +24,11 @@ def _instances():
     gens.append(synth.random_sparse(400, 3000, 7, 1000))
     gens.append(synth.random_sparse(150, 900, 9, 40))
     Rs = [32, 5, 16, 1, 3, 32, 7, 8, 2, 32, 17, 4, 9, 32, 6, 12, 33]
+    # unequal couplings of 1 and 4 bytes: what the packed kernel runs in groups
+    for k, R in enumerate((8, 16, 32, 17)):
+        gens += [synth.random_sparse(170 + 60 * k, 700 + 300 * k, 20 + k, 100),
+                 synth.random_sparse(210 + 40 * k, 900 + 200 * k, 30 + k, 5000)]
+        Rs += [R, R]
     items = []
     for k, (n, eu, ev, ew) in enumerate(gens):
         P = IsingProblem(n, eu, ev, ew)

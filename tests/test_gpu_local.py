@@ -51,12 +51,16 @@ def test_equals_the_planned_sweep_and_the_oracle(name, order, monkeypatch):
     arr = make()
     P = ResidualProblem.from_arrays(arr, flags=OPT_RESID_CLUSTER if order == "cluster" else 0)
     s = Schedule(20.0, 0.6, sweeps, 6, 11)
+    names = ["resid_local_cluster", "resid_cluster"] if order == "cluster" else ["resid_local"] + [f"resid_lockstep_{k}" for k in (1, 2, 3, 4)]
+    before = [sweep_launches(k) for k in names]
     monkeypatch.setenv("QB_RESID_KERNEL", "local")
     r = P.solve(s, R, 3, trace=True)
     u = P.solve(s, R, 3)   # without the trace: class barriers across sweeps too
     assert (u.branches() == r.branches()).all()
     monkeypatch.setenv("QB_RESID_KERNEL", order)
     o = P.solve(s, R, 3, trace=True)
+    ran = [sweep_launches(k) - b for k, b in zip(names, before)]
+    assert ran[0] == 2 and sum(ran[1:]) == (1 if order == "cluster" else (R + 63) // 64)
     monkeypatch.delenv("QB_RESID_KERNEL")
     X = r.branches()
     assert (X == o.branches()).all() and (r.marginals() == o.marginals()).all()

@@ -15,7 +15,7 @@ import numpy as np
 import pytest
 
 from oracle import oracle as O
-from qublar_b200 import (OPT_RESID_CLUSTER, Budget, IsingProblem, ResidualProblem, Schedule, branch_fractions, classify,
+from qublar_b200 import (OPT_RESID_CLUSTER, Budget, IsingProblem, ResidualProblem, Schedule, branch_fractions, classify, sweep_launches,
                          synth)
 
 pytestmark = pytest.mark.gpu
@@ -115,15 +115,20 @@ def test_residual_small_bit_exact():
 
 
 @pytest.mark.parametrize("R", [20, 40, 64], ids=["two_groups", "three_groups", "four_groups"])
-def test_residual_branch_groups_bit_exact(R):
+def test_residual_branch_groups_bit_exact(R, monkeypatch):
     """The lockstep sweep serves 16-branch groups with one compiled instance
     per group count: with 20, 40 and 64 branches (two, three and four
     groups), branches of every group equal the oracle's coloured-Philox run
-    of the same seed bit for bit."""
+    of the same seed bit for bit. (A pyramid of this size runs a CTA per branch
+    unless the lockstep sweep is asked for.)"""
     a = _small_tomo()
     P = ResidualProblem.from_arrays(a)
     s = Schedule(50.0, 1.0, 60, 20, 20)
+    monkeypatch.setenv("QB_RESID_KERNEL", "lockstep")
+    kernel = f"resid_lockstep_{(R + 15) // 16}"
+    before = sweep_launches(kernel)
     r = P.solve(s, R, 5)
+    assert sweep_launches(kernel) == before + 1
     X = r.branches()
     order, _ = P.colouring()
     temps = O.temperatures(s.t_hot, s.t_cold, s.anneal_sweeps, s.hold_sweeps)

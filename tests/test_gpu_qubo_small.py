@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from oracle import oracle as O
-from qublar_b200 import QuboProblem, Schedule, synth
+from qublar_b200 import QuboProblem, Schedule, sweep_launches, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -41,11 +41,13 @@ def test_equals_the_cooperative_sweep_and_the_oracle(name, monkeypatch):
          "ew": np.asarray(q["ew"], np.float32), "h": None if q["h"] is None else np.asarray(q["h"], np.float32)}
     P = QuboProblem.from_dict(q)
     s = Schedule(2.5, 0.1, 60, 7, 9)
+    before = sweep_launches("qubo_small"), sweep_launches("qubo_lockstep")
     monkeypatch.setenv("QB_QUBO_KERNEL", "small")
     r = P.solve(s, R, 2)
     t = P.solve(s, R, 2, trace=True)
     monkeypatch.setenv("QB_QUBO_KERNEL", "lockstep")
     o = P.solve(s, R, 2, trace=True)
+    assert (sweep_launches("qubo_small"), sweep_launches("qubo_lockstep")) == (before[0] + 2, before[1] + (R + 63) // 64)
     X = r.branches()
     assert (X == o.branches()).all() and (X == t.branches()).all()
     assert np.array_equal(r.energies(), o.energies())

@@ -23,32 +23,36 @@ def _sparse(n, m, wmax, seed):
 
 
 CASES = {
-    "k16": (lambda: synth.random_complete(16, 15, 3), 32, 60),
-    "two": (lambda: (2, np.array([0], np.int32), np.array([1], np.int32), np.array([5], np.int32)), 3, 20),
-    "er": (lambda: synth.erdos_renyi(300, 0.16, 2), 5, 80),
-    "dense_1000": (lambda: synth.random_complete(121, 1000, 7), 4, 60),
-    "dense_1e6": (lambda: synth.random_complete(65, 1000000, 7), 4, 60),
-    "dense_33": (lambda: synth.random_complete(33, 7, 1), 200, 30),
-    "dense_128": (lambda: synth.random_complete(128, 1, 2), 3, 30),
-    "dense_224": (lambda: synth.random_complete(224, 500, 2), 3, 17),
-    "dense_225": (lambda: synth.random_complete(225, 500, 2), 3, 9),
-    "torus": (lambda: synth.torus_pm1(30, 3), 7, 50),
-    "dense_many": (lambda: synth.random_complete(50, 1, 3), 700, 20),
-    "sparse_helpers": (lambda: _sparse(3001, 12000, 900, 5), 3, 40),
-    "sparse_many": (lambda: _sparse(2001, 9000, 100, 6), 100, 20),
-    "long_rows": (lambda: _sparse(9001, 180000, 3, 8), 2, 8),
+    "k16": (lambda: synth.random_complete(16, 15, 3), 32, 60, "ising_dense"),
+    "two": (lambda: (2, np.array([0], np.int32), np.array([1], np.int32), np.array([5], np.int32)), 3, 20, "ising_dense"),
+    "er": (lambda: synth.erdos_renyi(300, 0.16, 2), 5, 80, "ising_replica_w8"),
+    "er_no_helpers": (lambda: synth.erdos_renyi(300, 0.16, 2), 148, 20, "ising_replica_w8"),
+    "dense_1000": (lambda: synth.random_complete(121, 1000, 7), 4, 60, "ising_dense"),
+    "dense_1e6": (lambda: synth.random_complete(65, 1000000, 7), 4, 60, "ising_dense"),
+    "dense_33": (lambda: synth.random_complete(33, 7, 1), 200, 30, "ising_dense"),
+    "dense_128": (lambda: synth.random_complete(128, 1, 2), 3, 30, "ising_dense"),
+    "dense_224": (lambda: synth.random_complete(224, 500, 2), 3, 17, "ising_dense"),
+    "torus": (lambda: synth.torus_pm1(30, 3), 7, 50, "ising_replica_w8"),
+    "dense_many": (lambda: synth.random_complete(50, 1, 3), 700, 20, "ising_dense"),
+    "sparse_helpers": (lambda: _sparse(3001, 12000, 900, 5), 3, 40, "ising_replica_w32"),
+    "sparse_two_ctas": (lambda: _sparse(2001, 9000, 100, 6), 60, 20, "ising_replica_w8"),
+    "sparse_no_helpers": (lambda: _sparse(6001, 9000, 900, 6), 100, 12, "ising_replica_w32"),
+    "long_rows_w8": (lambda: synth.random_regular(2000, 100, 8), 2, 12, "ising_replica_w8_far"),
+    "long_rows_w32": (lambda: _sparse(801, 19000, 900, 8), 2, 12, "ising_replica_w32_far"),
 }
 
 
 @pytest.mark.parametrize("name", list(CASES))
 def test_equals_the_cta_per_replica_sweep_and_the_oracle(name, monkeypatch):
-    make, R, sweeps = CASES[name]
+    make, R, sweeps, kernel = CASES[name]
     g = make()
     P = IsingProblem(*g)
     s = P.scaled_schedule(sweeps, 3)
+    before = sweep_launches(kernel), sweep_launches("ising_fields")
     r = P.solve(s, R, 9, trace=True)
     monkeypatch.setenv("QB_ISING_THREADS", "512")
     o = P.solve(s, R, 9, trace=True)
+    assert (sweep_launches(kernel), sweep_launches("ising_fields")) == (before[0] + 1, before[1] + 1)
     monkeypatch.delenv("QB_ISING_THREADS")
     assert (r.branches() == o.branches()).all() and (r.fields() == o.fields()).all()
     assert (r.energies_tracked() == o.energies_tracked()).all() and (r.energies() == o.energies()).all()
@@ -62,12 +66,16 @@ def test_equals_the_cta_per_replica_sweep_and_the_oracle(name, monkeypatch):
         assert (r.branches()[k] == x).all() and r.energies_tracked()[k] == e
 
 
-@pytest.mark.parametrize("t", [1e-3, 0.7, 4095.0, 4097.0, 3e7, 1e13, 1e16])
+@pytest.mark.parametrize("t", [1e-3, 0.7, 4095.0, 4097.0, 3e7, 2.0 ** 39, 2.0 ** 40, 1.0001 * 2.0 ** 40, 1e16])
 def test_temperatures_of_every_size(t, monkeypatch):
+    """Both precisions of the limit's logarithm; above 2^40 the CTA-per-replica sweep."""
     g = synth.random_complete(40, 20000, 1)
     P = IsingProblem(*g)
     s = Schedule(t, t / 3, 25, 2, 0)
+    kernel = "ising_dense" if t <= 2.0 ** 40 else "ising_fields"
+    before = sweep_launches(kernel)
     r = P.solve(s, 6)
+    assert sweep_launches(kernel) == before + 1
     monkeypatch.setenv("QB_ISING_THREADS", "64")
     o = P.solve(s, 6)
     assert (r.branches() == o.branches()).all() and (r.energies_tracked() == o.energies_tracked()).all()

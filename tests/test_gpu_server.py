@@ -3,7 +3,7 @@
 Each result must be the same alone and in the mix: a request's branches equal
 qb_solve's for the same problem, schedule and seeds, bit for bit, whatever the
 server runs beside it (ising requests share ticks of the packed kernel,
-residual requests run as cluster launches beside them). Admission respects the
+requests whose sweep has no grid barrier run beside them). Admission respects the
 device-memory budget, requests admitted while others run finish without
 waiting for them, cancellation and timeouts behave as declared.
 """
@@ -27,7 +27,9 @@ RESID = OPT_DEFER_UPLOAD | OPT_RESID_CLUSTER
 def _ising_cases():
     gens = [g for _, g in synth.mixed_batch(6, seed=21, n_min=100, n_max=4000)]
     gens.append(synth.random_sparse(500, 4000, 3, 1000))   # int32 weights
-    gens.append(synth.torus_pm1(150, 5))                    # 22,500 bits: global state in a 96 KiB CTA
+    gens.append(synth.torus_pm1(150, 5))                    # 22,500 bits: words in a CTA
+    n, eu, ev, ew = synth.torus_pm1(150, 6)                  # unequal couplings: global state in a 96 KiB CTA
+    gens.append((n, eu, ev, ew * (1 + np.arange(ew.size, dtype=np.int32) % 3)))
     out = []
     for k, g in enumerate(gens):
         P0 = IsingProblem(*g)
@@ -190,27 +192,41 @@ def test_cancel_and_timeout():
     S.close()
 
 
-def test_graph_and_direct_ticks_agree():
-    g = synth.random_regular(1500, 12, 8)
+@pytest.mark.parametrize("couplings", ["unequal", "one size"])
+def test_graph_and_direct_ticks_agree(couplings):
+    """Ticks of the packed kernel (unequal couplings) replayed from a captured
+    graph and launched directly; word units are launched directly in both."""
+    n, eu, ev, ew = synth.random_regular(1500, 12, 8)
+    if couplings == "unequal":
+        ew = (ew * (1 + np.arange(ew.size) % 5)).astype(np.int32)
     sched = Schedule(3.0, 0.05, 200, 20, 0)
     out = []
     for use_graph in (True, False):
+        kernel = "ising_word_16" if couplings == "one size" else "ising_batch_replay" if use_graph else "ising_batch"
+        before = sweep_launches(kernel)
         S = Server(use_graph=use_graph, tick_target_us=1000)
-        P = IsingProblem(*g, flags=DEFER)   # must outlive its request
+        P = IsingProblem(n, eu, ev, ew, flags=DEFER)   # must outlive its request
         rid = S.submit(P, sched, 16, 4)
         S.wait(rid, 120000)
         out.append(S.branches(rid))
-        assert S.stats().ticks > 1
+        assert S.stats().ticks > 1 and sweep_launches(kernel) == before + S.stats().ticks
         S.close()
     assert (out[0] == out[1]).all()
 
 
-def test_exclusive_requests_beside_ticks_are_the_same_alone():
+@pytest.mark.parametrize("sweeps", ["lockstep", "in a CTA"])
+def test_exclusive_requests_beside_ticks_are_the_same_alone(sweeps, monkeypatch):
     """With coop_parts = 1 a lockstep-planned pyramid and a weighted QUBO run
-    as whole-device sweeps with nothing beside them; ising requests submitted
-    around them still finish, and every result equals its solve alone."""
+    with nothing beside them, as whole-device sweeps or (as small as these) with
+    a branch to a CTA; ising requests submitted around them still finish, and
+    every result equals its solve alone."""
+    if sweeps == "lockstep":
+        monkeypatch.setenv("QB_RESID_KERNEL", "lockstep")
+        monkeypatch.setenv("QB_QUBO_KERNEL", "lockstep")
+    kernels = ["resid_lockstep_2", "qubo_lockstep"] if sweeps == "lockstep" else ["resid_local", "qubo_small"]
+    before = [sweep_launches(k) for k in kernels]
     pyr = synth.tomography(synth.small_tomo_params(0.2, 24))
-    q = synth.random_qubo(400, 2500, 17)
+    q = synth.random_qubo(*((400, 2500) if sweeps == "lockstep" else (200, 1500)), 17)
     g1, g2 = synth.random_regular(2000, 8, 5), synth.torus_pm1(40, 2)
     sp, sq, si = Schedule(50.0, 1.0, 60, 15, 25), Schedule(3.0, 0.05, 120, 10, 32), Schedule(3.0, 0.05, 200, 0, 0)
     P1 = IsingProblem(*g1, flags=DEFER)
@@ -221,6 +237,7 @@ def test_exclusive_requests_beside_ticks_are_the_same_alone():
     ids = [S.submit(P1, si, 16, 1), S.submit(Pp, sp, 20, 2), S.submit(Pq, sq, 40, 3), S.submit(P2, si, 8, 4)]
     for i in ids:
         S.wait(i, 120000)
+    assert [sweep_launches(k) for k in kernels] == [b + 1 for b in before]
     infos = [S.info(i) for i in ids]
     # nothing overlaps an exclusive request
     for k in (1, 2):
@@ -235,11 +252,16 @@ def test_exclusive_requests_beside_ticks_are_the_same_alone():
     S.close()
 
 
-def test_cooperative_requests_overlap_on_partitions_and_match_alone():
+def test_cooperative_requests_overlap_on_partitions_and_match_alone(monkeypatch):
     """Lockstep pyramids and weighted QUBOs run side by side on partitions of
     the device (a deferred pyramid is planned again for its partition's grid
     at submission), beside ising ticks; at least two of them overlap in time,
-    and every result equals its solve alone on the whole device."""
+    and every result equals its solve alone on the whole device. (Problems of
+    these sizes keep a branch in one CTA unless the lockstep sweeps are asked for.)"""
+    monkeypatch.setenv("QB_RESID_KERNEL", "lockstep")
+    monkeypatch.setenv("QB_QUBO_KERNEL", "lockstep")
+    kernels = ["resid_lockstep_1", "resid_lockstep_2", "qubo_lockstep"]
+    before = [sweep_launches(k) for k in kernels]
     pyrs = [synth.tomography(synth.small_tomo_params(0.2 + 0.02 * k, 24)) for k in range(3)]
     qs = [synth.random_qubo(400 + 100 * k, 2500, 17 + k) for k in range(2)]
     g1 = synth.random_regular(2000, 8, 5)
@@ -253,6 +275,7 @@ def test_cooperative_requests_overlap_on_partitions_and_match_alone():
     ids.append(S.submit(Pi, si, 16, 20))
     for i in ids:
         S.wait(i, 300000)
+    assert [sweep_launches(k) for k in kernels] == [before[0] + 1, before[1] + 2, before[2] + 2]
     infos = [S.info(i) for i in ids]
     coop = infos[:5]
     overlaps = sum(1 for a in range(5) for b in range(a + 1, 5)

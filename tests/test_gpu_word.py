@@ -43,7 +43,9 @@ def test_words_equal_the_oracle(name, R):
     g = GRAPHS[name]()
     P = IsingProblem(*g)
     s = P.scaled_schedule(30, 4)
+    before = sweep_launches("ising_word_16")
     B = solve_batch([(P, s, R, 6)])
+    assert sweep_launches("ising_word_16") == before + 1
     X, E, F = B.branches(0), B.energies_tracked(0), B.fields(0)
     G = O.Graph(*g)
     order, _ = P.colouring()
@@ -78,13 +80,17 @@ def test_every_unit_width_equals_the_oracle(name, R):
     B.close()
 
 
-@pytest.mark.parametrize("n", [32767, 32769])
-def test_both_adjacency_widths_equal_the_field_sweep(n):
+@pytest.mark.parametrize("n", [32767, 32768, 32769])
+def test_both_adjacency_widths_equal_the_field_sweep(n, monkeypatch):
     g = synth.random_regular(n, 5, 11)
     P = IsingProblem(*g)
     s = P.scaled_schedule(8, 1)
+    kernel = "ising_word_16" if n <= 32768 else "ising_word_32"
+    before = sweep_launches(kernel), sweep_launches("ising_fields")
     B = solve_batch([(P, s, 10, 0)])
+    monkeypatch.setenv("QB_ISING_THREADS", "512")
     r = P.solve(s, 10)
+    assert (sweep_launches(kernel), sweep_launches("ising_fields")) == (before[0] + 1, before[1] + 1)
     assert (B.branches(0) == r.branches()).all()
     assert (B.energies_tracked(0) == r.energies_tracked()).all() and (B.fields(0) == r.fields()).all()
 
@@ -94,9 +100,11 @@ def test_many_replicas_equal_the_cta_per_replica_sweep(R, monkeypatch):
     g = synth.random_regular(331, 21, 2)
     P = IsingProblem(*g)
     b = Budget(6.0, 0.2, 40, 3)
+    before = sweep_launches("ising_word_16"), sweep_launches("ising_fields")
     r = P.solve(b, R, 4)
     monkeypatch.setenv("QB_ISING_THREADS", "128")
     o = P.solve(b, R, 4)
+    assert (sweep_launches("ising_word_16"), sweep_launches("ising_fields")) == (before[0] + 1, before[1] + 1)
     assert (r.branches() == o.branches()).all() and (r.fields() == o.fields()).all()
     assert (r.energies_tracked() == o.energies_tracked()).all() and (r.energies() == o.energies()).all()
 
@@ -106,11 +114,13 @@ def test_whole_device_words_equal_the_field_sweep(n, d, R, monkeypatch):
     """Large graphs of few classes: words in global memory on a cooperative grid."""
     g = synth.random_regular(n, d, 3) if n != 90000 else synth.torus_pm1(300, 5)
     P = IsingProblem(*g)
-    assert P.n >= 2000 * P.info().n_colours
     s = P.scaled_schedule(9, 1)
+    kernel = "ising_grid_16" if P.n <= 32768 else "ising_grid_32"
+    before = sweep_launches(kernel), sweep_launches("ising_fields")
     r = P.solve(s, R, 12)
     monkeypatch.setenv("QB_ISING_THREADS", "512")
     o = P.solve(s, R, 12)
+    assert (sweep_launches(kernel), sweep_launches("ising_fields")) == (before[0] + 1, before[1] + 1)
     assert (r.branches() == o.branches()).all() and (r.fields() == o.fields()).all()
     assert (r.energies_tracked() == o.energies_tracked()).all() and (r.energies() == o.energies()).all()
     assert (r.marginals() == o.marginals()).all()
