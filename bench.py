@@ -333,17 +333,17 @@ def run_batch(args):
                                                          "max_group": cfg.max_group},
                    "work_items": infos[0].work_items, "global_items": infos[0].global_items,
                    "l2": "flushed (256 MB write) before every timed step", "parallelism": "1 GPU"},
-        "plain": {"value": plain, "unit": "attempts/s", "form": "one qb_solve per instance (CTA per replica)",
+        "plain": {"value": plain, "unit": "attempts/s", "form": "one qb_solve per instance",
                   "sample": f"{len(sample)} instances stratified by size"},
         "vs_plain": value / plain,
         "e2e": {"value": attempts / e2e_s, "unit": "attempts/s", "h2d_bytes_per_step": int(h2d),
                 "d2h_bytes_per_step": int(d2h), "s_per_step": e2e_s},
         "gpu_launches": sum(i.launches for i in infos),
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
-                     "peak_kind": peak_kind, "traffic": None, "kernel": "ising_batch_kernel",
+                     "peak_kind": peak_kind, "traffic": None, "kernel": "ising_word_kernel",
                      "kernel_ms": anneal_ms, "algorithmic_bytes": alg,
                      "note": "CSR and state stay in L2 and shared memory; the sweep is issue-bound (Philox, "
-                             "shared-memory field updates), not DRAM-bound"},
+                             "neighbour counts), not DRAM-bound"},
         "clocks": clocks,
     }
     if not args.no_cpu_baseline:
@@ -549,9 +549,9 @@ def serve_measure(n_requests, rates=(0.5, 0.8), plain_sample=24, warm=3):
 
 
 SERVE_POLICY = (f"pyramids >= {SERVE_LOCKSTEP_BITS} bits: lockstep sweep on one of 4 SM partitions, side by side; "
-                "smaller pyramids: one cluster per branch; Max-Cut >= "
+                "smaller pyramids: one CTA or cluster per branch; Max-Cut >= "
                 f"{SERVE_QUBO_MAXCUT_BITS} bits: the equal weighted QUBO on a partition; smaller Max-Cut: ticks of "
-                "the packed kernel")
+                "word units")
 
 
 def run_serve(args):
@@ -567,7 +567,7 @@ def run_serve(args):
         "latency": m["latency"],
         "plain": {"value": m["plain"], "unit": "attempts/s",
                   "form": "each request alone through qb_solve (lockstep sweep for pyramids, the whole-device "
-                          f"QUBO sweep for Max-Cut >= {SERVE_QUBO_MAXCUT_BITS} bits, CTA per replica below)",
+                          f"QUBO sweep for Max-Cut >= {SERVE_QUBO_MAXCUT_BITS} bits, its own sweep below)",
                   "sample": f"{m['plain_sample']} requests"},
         "vs_plain": m["vs_plain"],
         "equal_energy": m["equal_energy"],

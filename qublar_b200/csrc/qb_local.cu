@@ -138,7 +138,8 @@ __global__ void __launch_bounds__(kLocalThreads, 1) resid_local_kernel(ResidLoca
     // coefficient; entries past the segment are the zero pair rho[nr] with a
     // zero coefficient, which change nothing. na, nb: the next item's record.
     // issue() starts the loads and makes the draw, nothing in it waits for
-    // them: it runs ahead of the barrier, whose wait hides them.
+    // them: it runs ahead of the barrier, whose wait hides them for every warp
+    // but the class's last, whose arrival comes behind it.
     uint4 ra{}, rb{}, na{}, nb{};
     uint2 en[kHold];
     int nbr[kNbrLane];

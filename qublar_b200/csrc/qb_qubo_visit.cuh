@@ -1,6 +1,8 @@
-// Device code of a weighted-QUBO visit shared by the sweeps (qb_qubo.cu,
-// qb_qubo_local.cu): a warp visits one bit for 64 replicas, lane l serves
-// replicas l and l + 32.
+// Device code of a weighted-QUBO visit. Both sweeps (qb_qubo.cu,
+// qb_qubo_local.cu) add flips by two_sum_acc; the walk over the flipped
+// neighbours is the cooperative sweep's: a warp visits one bit for 64 replicas,
+// lane l serves replicas l and l + 32 (the small sweep, 32 replicas to a warp,
+// adds every flipped neighbour to all of them, masked).
 #pragma once
 
 #include <cuda_runtime.h>

@@ -1,5 +1,5 @@
-// Integer Ising sweep of few replicas: a CTA anneals one replica with the
-// random part of every decision taken off the sweep's chain.
+// Integer Ising sweep of few replicas, or of a dense graph: a CTA anneals one
+// replica with the random part of every decision taken off the sweep's chain.
 //
 // With no more replicas than SMs the time is the chain of colour classes
 // (ER(800, 0.06): 17 classes x 1000 sweeps), not the work. So
@@ -14,9 +14,9 @@
 //     loaded before the barrier that opens its class, as is the CSR (in shared
 //     memory where it fits).
 //
-// Bound: the dependent instructions of a class step in one warp (ncu: 90 warp
-// instructions per consumer warp and class, 44 % issue, barrier and fixed
-// latencies; about 0.5 us against 0.74 of ising_anneal_kernel). Kernel time on
+// Bound: the dependent instructions of a class step in one warp (ncu, ER(800,
+// 0.06), 16 replicas: 29 % issue on the SMs in use, barrier and fixed latencies;
+// about 0.5 us against 0.74 of ising_anneal_kernel). Kernel time on
 // a B200, before and after: ER(800, 0.06), 16 replicas x 1000 sweeps 12.4 and
 // 8.5 ms; 3,001 bits of degree 8 with 32-bit couplings, 50 x 400: 2.4 and 1.8;
 // complete graph of 16 spins, 32 x 100 (ising_dense_kernel below): 0.78 and
@@ -318,9 +318,9 @@ __global__ void __launch_bounds__(32 * kReplicaWarps, 1) ising_replica_kernel(Re
 // in registers, lane l the fields of bits l, l + 32, ..., and visits the bits
 // one by one in sweep order (the order inside a class does not matter), with
 // the coupling matrix in shared memory. A visit is a multiply, a compare, a
-// shuffle of the flip and a multiply-add: about 50 cycles, against a class
-// step of one bit through shared memory (about 500). The other warps draw the
-// limits kDenseAhead sweeps at a time.
+// shuffle of the flip and a multiply-add: 50 to 95 ns by the bits a lane holds,
+// against a class step through shared memory of 0.5 us and more. The other warps
+// draw the limits kDenseAhead sweeps at a time.
 constexpr int kDenseAhead = 8;
 constexpr int kDenseMax = 224;   // bits: the matrix of 4-byte couplings fits shared memory
 
@@ -418,8 +418,8 @@ __global__ void __launch_bounds__(128) ising_dense_kernel(ReplicaArgs A) {
     if (lane == 0) A.e_out[rep] = E;
 }
 
-// A visit costs about an eighth of a class step: dense graphs, where most
-// classes hold a few bits.
+// A visit costs about an eighth of a class step: dense graphs, where most classes
+// hold a few bits (above one replica per SM the route weighs its waves).
 bool dense_fit(const IsingPlan& p) { return p.n <= kDenseMax && p.n <= 8 * p.col.n_colours(); }
 size_t dense_smem(const IsingPlan& p) {
     return (size_t(p.n) * size_t(p.n) + 2 * size_t(kDenseAhead) * size_t(p.n)) * 4;

@@ -1,7 +1,7 @@
 // The route of a single integer solve: estimates of a solve's microseconds on a
 // B200 for each kernel that can serve it, fitted to measured kernel times over
 // 25 to 60,000 bits, degrees 3 to 450 and 149 to 8,192 replicas (497 points; the
-// choice costs 0.4 % over the best kernel on average, at most 30 %; the wrong
+// choice costs 0.5 % over the best kernel on average, at most 30 %; the wrong
 // kernel up to 8 times).
 #include <algorithm>
 #include <cmath>

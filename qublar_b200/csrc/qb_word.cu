@@ -12,12 +12,13 @@
 // bit positions, and popcounts give the pair's counts.
 //
 // Bound: instruction issue, the half-rate integer pipe above all (ncu: 54 % of
-// it, 59 % issue; 256 warp instructions per 64 proposals of degree 48, a
-// quarter of them the Philox block, 25 per 16 neighbours). The field-carrying
+// it, 59 % issue in units of 16 replicas, 51 and 56 in units of 32; 240 warp
+// instructions per 64 proposals of degree 48, a quarter of them the Philox block,
+// 25 per 16 neighbours). The field-carrying
 // form (qb_batch.cu) spends an atomic per flipped neighbour and replica, and 5
 // bytes of state per replica and bit against 1/4 here. Measured on a B200,
 // kernel time: 4096 replicas x 300 sweeps of ER(800, 0.06) 16.6 ms with a CTA
-// per replica, 6.3 ms here; 128 mixed tori and d-regular graphs of 200 to
+// per replica, 6.4 ms here; 128 mixed tori and d-regular graphs of 200 to
 // 20,000 bits, 32 replicas x 200 sweeps, 50 ms packed, 21.6 ms here (1.8e11
 // proposals/s; 2.2e11 on 1,024 instances up to 5,000 bits).
 //
